@@ -24,8 +24,7 @@ __device__ __forceinline__ float2 gather_point(const float2 *__restrict__ patch,
                                                float t1, float t2, const WinPoly &wp) {
     constexpr int W = 2 * K + 1;
     float w1[W], w2[W];
-    weights_poly<K>(t1, w1, wp);
-    weights_poly<K>(t2, w2, wp);
+    weights_poly2<K>(t1, t2, w1, w2, wp);
     const float2 *base = patch + lr * PC + lc + (Ke - K);
     float sx = 0.f, sy = 0.f, ex = 0.f, ey = 0.f;
 #pragma unroll
@@ -71,8 +70,7 @@ __device__ __forceinline__ float2 gather_direct_f32(const float2 *__restrict__ g
     constexpr int W = 2 * K + 1;
     constexpr int V = K + 1;  // float4 loads per row
     float w1[W], w2[W];
-    weights_poly<K>(t1, w1, wp);
-    weights_poly<K>(t2, w2, wp);
+    weights_poly2<K>(t1, t2, w1, w2, wp);
     const int col0 = mu2 + H - K;
     const int odd = col0 & 1;
     float ws[2 * V];
@@ -281,8 +279,7 @@ __device__ __forceinline__ void spread_item(const Rec32 *__restrict__ recs, int 
             const int st = lc / S::SW;
             my_key = (st << 4) | lr;
             float w1[W], w2[W];
-            weights_poly<K>(__int_as_float(raw.x), w1, wp);
-            weights_poly<K>(__int_as_float(raw.y), w2, wp);
+            weights_poly2<K>(__int_as_float(raw.x), __int_as_float(raw.y), w1, w2, wp);
             float *sp = scr + lane * SP;
             const int q = lc - st * S::SW;  // first patch column of the point within the strip
             reinterpret_cast<int4 *>(sp)[0] = make_int4(lr, q, st, 0);
