@@ -30,6 +30,7 @@
 #include "nfft2d_device.cuh"
 #include "nfft2d_internal.h"
 #include "nfft2d_kargs.cuh"
+#include "nfft2d_tc.cuh"
 #include "nfft2d_tile_ops.cuh"
 
 using namespace nfft2d;
@@ -54,7 +55,9 @@ struct alignas(128) BatchDesc {
     int row_base;       // first global oversampled row (pad / halo kernels)
     int crop_base;      // first global output row (crop)
     int chunk;          // maximum points per work item
-    int point_base;     // first global point of this transform (direct gather)
+    int point_base;     // points of the transforms before this one that the direct gather serves
+    int points;         // this transform's points
+    int tc;             // the tensor-core gather serves it
 };
 
 struct BatchIO {
@@ -192,11 +195,11 @@ __global__ void k_batch_fold(const BatchDesc *__restrict__ d) {
 }
 
 // ---- gather over the points of all transforms --------------------------
-// Direct gather over all transforms: one thread per binned point, the
-// transform found by its global point index; taps read straight from that
-// transform's padded grid (the single-plan FP32 direct gather).
+// Direct gather: one thread per binned point, the transform found by its
+// index among the points of the transforms it serves; taps read straight from
+// that transform's padded grid (the single-plan FP32 direct gather).
 // One launch per window width: transforms [first, first + n) of the batch's
-// internal order share K and hold global points [point0, point0 + npoints).
+// internal order share K and hold points [point0, point0 + npoints).
 template <int K>
 __global__ void __launch_bounds__(kThreads, K <= 6 ? 4 : 3)  // as the single-plan FP32 gather
     k_batch_gather_direct(const BatchDesc *__restrict__ d, int first, int n, const BatchIO *__restrict__ io,
@@ -214,6 +217,32 @@ __global__ void __launch_bounds__(kThreads, K <= 6 ? 4 : 3)  // as the single-pl
     }
     io[t].out[raw.w] = gather_direct_f32<K, true>(D.grid, __ldg(&D.g.H), __ldg(&D.g.C), mu1, mu2, __int_as_float(raw.x),
                                             __int_as_float(raw.y), wp);
+}
+
+// The other transforms of a width on the tensor cores (as k_gather_tc): every
+// CTA walks its share of each one's work items; the shares are dealt from a
+// CTA that moves on with the items, so that short lists fall on different CTAs.
+template <int K>
+__global__ void __launch_bounds__(kTcPoints, kTcCtas)
+    k_batch_gather_tc(const BatchDesc *__restrict__ d, int first, int n, const BatchIO *__restrict__ io,
+                      const __grid_constant__ WinPoly wp, int *status) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    TcGather<K> t;
+    t.begin(smem_raw, &tmem_slot, &bar);
+    unsigned turn = blockIdx.x;
+    for (int i = first; i < first + n; ++i) {
+        const BatchDesc &D = d[i];
+        if (!D.tc) continue;
+        const int group = max(1, min(16, D.n_chunks / static_cast<int>(8 * gridDim.x)));  // as tc_run_items
+        if (!t.template run<true>(TcWalk(D.chunks, D.n_chunks, group, D.g), static_cast<int>(turn) * group, D.grid, D.g,
+                                  D.recs, D.points, io[i].out, 0, wp, status))
+            break;
+        const unsigned runs = (D.n_chunks + group - 1) / group;
+        turn = (turn + gridDim.x - runs % gridDim.x) % gridDim.x;
+    }
+    t.end();
 }
 
 // ---- persistent spread over the work items of all transforms --------------
@@ -290,7 +319,8 @@ struct nfft2d_batch_s {
     struct KGroup {
         int K = 6, first = 0, n = 0;
         int chunk0 = 0, total_chunks = 0;  // their global work items
-        int point0 = 0, total_points = 0;  // their global points
+        int point0 = 0, total_points = 0;  // the direct gather's points among them
+        bool tc = false;                   // some are the tensor-core gather's
         Geom g0{};                         // patch geometry of the width
         WinPoly poly{};                    // window polynomials of the width
     };
@@ -348,7 +378,15 @@ int run_ffts(nfft2d_batch_s *b, int dir) {
 }
 
 template <int K>
-int launch_gather(nfft2d_batch_s *b, const nfft2d_batch_s::KGroup &kg) {
+int launch_gather(nfft2d_batch_s *b, const nfft2d_batch_s::KGroup &kg, int sms) {
+    if constexpr (K >= 6) {
+        if (kg.tc) {
+            B_TRY(cudaFuncSetAttribute(k_batch_gather_tc<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcGeo<K>::SMEM));
+            k_batch_gather_tc<K><<<kTcCtas * sms, kTcPoints, TcGeo<K>::SMEM, b->stream>>>(b->d_desc, kg.first, kg.n, b->d_io,
+                                                                                         kg.poly, b->d_status);
+            B_TRY(cudaGetLastError());
+        }
+    }
     if (kg.total_points == 0) return NFFT2D_OK;
     k_batch_gather_direct<K><<<(kg.total_points + kThreads - 1) / kThreads, kThreads, 0, b->stream>>>(
         b->d_desc, kg.first, kg.n, b->d_io, kg.point0, kg.total_points, kg.poly, b->d_status);
@@ -375,15 +413,15 @@ int launch_spread(nfft2d_batch_s *b, const nfft2d_batch_s::KGroup &kg, int sms) 
     return NFFT2D_OK;
 }
 
-int launch_gather_k(nfft2d_batch_s *b, const nfft2d_batch_s::KGroup &kg) {
+int launch_gather_k(nfft2d_batch_s *b, const nfft2d_batch_s::KGroup &kg, int sms) {
     switch (kg.K) {
-        case 2: return launch_gather<2>(b, kg);
-        case 3: return launch_gather<3>(b, kg);
-        case 4: return launch_gather<4>(b, kg);
-        case 5: return launch_gather<5>(b, kg);
-        case 6: return launch_gather<6>(b, kg);
-        case 7: return launch_gather<7>(b, kg);
-        case 8: return launch_gather<8>(b, kg);
+        case 2: return launch_gather<2>(b, kg, sms);
+        case 3: return launch_gather<3>(b, kg, sms);
+        case 4: return launch_gather<4>(b, kg, sms);
+        case 5: return launch_gather<5>(b, kg, sms);
+        case 6: return launch_gather<6>(b, kg, sms);
+        case 7: return launch_gather<7>(b, kg, sms);
+        case 8: return launch_gather<8>(b, kg, sms);
         default: return NFFT2D_ERR_INVALID_ARG;
     }
 }
@@ -418,7 +456,7 @@ int enqueue(nfft2d_batch_s *b, int type) {
         k_batch_fill<<<dim3(16, n), kThreads, 0, b->stream>>>(b->d_desc);
         B_TRY(cudaGetLastError());
         for (const auto &kg : b->kgroups)
-            if ((st = launch_gather_k(b, kg)) != NFFT2D_OK) return st;
+            if ((st = launch_gather_k(b, kg, sms)) != NFFT2D_OK) return st;
     } else {
         B_TRY(cudaMemsetAsync(b->grids, 0, b->grid_bytes, b->stream));
         int st;
@@ -656,7 +694,7 @@ int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *cons
     }
     std::vector<BatchDesc> h(b->count);
     int chunks = 0, rows = 0, crop = 0;
-    long long points = 0;
+    long long points = 0, all_points = 0;
     for (int i = 0; i < b->count; ++i) {
         nfft2d_plan_s *p = b->plans[i];
         BatchDesc &D = h[i];
@@ -676,22 +714,27 @@ int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *cons
         D.crop_base = crop;
         D.chunk = p->chunk;
         D.point_base = static_cast<int>(points);
-        points += p->M;
+        D.points = static_cast<int>(p->M);
+        D.tc = tc_gather_pays(p->K, p->g, p->M);
+        if (!D.tc) points += p->M;
+        all_points += p->M;
         chunks += D.n_chunks;
         rows += p->g.n1;
         crop += p->N1;
     }
     B_TRY(cudaMemcpy(b->d_desc, h.data(), sizeof(BatchDesc) * b->count, cudaMemcpyHostToDevice));
-    if (points > 0x7fffffffLL) return NFFT2D_ERR_INVALID_ARG;  // global point indices are int
+    if (all_points > 0x7fffffffLL) return NFFT2D_ERR_INVALID_ARG;  // global point indices are int
     for (auto &kg : b->kgroups) {
         kg.chunk0 = h[kg.first].chunk_base;
         kg.point0 = h[kg.first].point_base;
         const int last = kg.first + kg.n - 1;
         kg.total_chunks = h[last].chunk_base + h[last].n_chunks - kg.chunk0;
-        kg.total_points = static_cast<int>(h[last].point_base + b->plans[last]->M - kg.point0);
+        kg.total_points = static_cast<int>(h[last].point_base + (h[last].tc ? 0 : b->plans[last]->M) - kg.point0);
+        kg.tc = false;
+        for (int i = kg.first; i <= last; ++i) kg.tc = kg.tc || h[i].tc;
     }
     b->total_chunks = chunks;
-    b->total_points = static_cast<int>(points);
+    b->total_points = static_cast<int>(all_points);
     b->total_rows = rows;
     b->total_crop = crop;
     b->points_valid = true;

@@ -17,14 +17,18 @@
 // DIRECT variant (both precisions): one thread per sorted point reads its
 // taps straight from the padded grid (L1/L2), no shared memory.  FP32 plans
 // use k_gather_direct_f32 / k_grad_direct_f32 (two taps per 16-byte load,
-// bounded registers, compensated row sum in the gather); FP64 plans the
-// generic k_gather_direct.
+// bounded registers, compensated row sum in the gather), the gather of dense
+// sets and wide windows k_gather_tc (tc_gather_pays); FP64 plans the generic
+// k_gather_direct.
 #include <cuda.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "nfft2d_device.cuh"
 #include "nfft2d_internal.h"
 #include "nfft2d_kargs.cuh"
+#include "nfft2d_tc.cuh"
 #include "nfft2d_tile_ops.cuh"
 
 namespace nfft2d {
@@ -283,6 +287,29 @@ __global__ void __launch_bounds__(kThreads, K <= 6 ? 4 : 3)
                                 : gather_direct_f32<K, false>(grid, g.H, g.C, mu1, mu2, r.t1, r.t2, a.poly);
 }
 
+// The direct gather's results from the tensor cores (nfft2d_tc.cuh), for
+// dense sets and wide windows: persistent CTAs over the work items, four to an
+// SM (their accumulators fill its tensor memory).  Bound by shared memory:
+// operand reads of the MMAs, 4 cycles a point, and the point's own weights
+// going in and out, 5 of the 12 cycles it takes an SM at w 6 (ncu, 2^23
+// clustered points: issue 48 %, load/store wavefronts 54 %); the direct gather
+// takes 16.7, bound by L1.  2^22 uniform points, w 6: 268 -> 213 us; 2^24
+// clustered: 960 -> 812 us.
+template <int K, bool COMP>
+__global__ void __launch_bounds__(kTcPoints, kTcCtas)
+    k_gather_tc(const float2 *__restrict__ grid, const Rec32 *__restrict__ recs, const int4 *__restrict__ chunks,
+                float2 *__restrict__ out, int group, const __grid_constant__ KArgs a) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    const int n = a.n_chunks >= 0 ? a.n_chunks : a.status[0];  // < 0: counted on the device only
+    TcGather<K> t;
+    t.begin(smem_raw, &tmem_slot, &bar);
+    t.template run<COMP>(TcWalk(chunks, n, group, a.g), blockIdx.x * group, grid, a.g, recs, a.M, out, a.binned_io,
+                         a.poly, a.status);
+    t.end();
+}
+
 // The FP32 coordinate gradient with the forward gather's 16-byte row loads:
 // per row the value and slope column weights (shifted by one for odd starts,
 // as in gather_direct_f32) give the partials r = sum w2 v and q = sum dw2 v;
@@ -378,6 +405,19 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
             static_cast<const double2 *>(p->grid), static_cast<const Rec64 *>(p->recs), static_cast<double2 *>(f),
             static_cast<const double2 *>(v), static_cast<double *>(g1), static_cast<double *>(g2), a);
     } else if constexpr (MODE == 0) {
+        if constexpr (K >= 6) {
+            if (tc_gather_pays(K, p->g, p->M)) {
+                const long long items = p->n_chunks >= 0 ? p->n_chunks : p->chunks_cap;
+                auto kernel = p->compensated ? k_gather_tc<K, true> : k_gather_tc<K, false>;
+                const cudaError_t e = prepare_smem(kernel, TcGeo<K>::SMEM);
+                if (e != cudaSuccess) return e;
+                const long long ctas = std::min<long long>(items, static_cast<long long>(kTcCtas) * p->num_sms);
+                kernel<<<static_cast<unsigned>(ctas), kTcPoints, TcGeo<K>::SMEM, p->stream>>>(
+                    static_cast<const float2 *>(p->grid), static_cast<const Rec32 *>(p->recs), p->chunks,
+                    static_cast<float2 *>(f), tc_run_items(items, ctas), a);
+                return cudaGetLastError();
+            }
+        }
         k_gather_direct_f32<K><<<blocks, kThreads, 0, p->stream>>>(
             static_cast<const float2 *>(p->grid), static_cast<const Rec32 *>(p->recs), static_cast<float2 *>(f), a);
     } else {
