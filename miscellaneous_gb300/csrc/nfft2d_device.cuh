@@ -144,35 +144,9 @@ __device__ __forceinline__ void weights_f32(float t, float (&w)[2 * K + 1], floa
     }
 }
 
-// All 2K+1 taps from the plan's polynomials: Horner steps on FP32 FMAs whose
-// coefficients are read from kernel parameter space (uniform across the warp).
-// Taps (2j, 2j+1) share one packed FP32x2 FMA (__ffma2_rn) per Horner step;
-// the odd last tap runs alone.
-template <int K>
-__device__ __forceinline__ void weights_poly(float t, float (&w)[2 * K + 1], const WinPoly &P) {
-    constexpr int D = poly_degree(K);
-    const float2 tt = make_float2(t, t);
-    float2 acc[K];
-    float last = P.c[D][2 * K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) acc[j] = *reinterpret_cast<const float2 *>(&P.c[D][2 * j]);
-#pragma unroll
-    for (int d = D - 1; d >= 0; --d) {
-#pragma unroll
-        for (int j = 0; j < K; ++j) acc[j] = __ffma2_rn(acc[j], tt, *reinterpret_cast<const float2 *>(&P.c[d][2 * j]));
-        last = fmaf(last, t, P.c[d][2 * K]);
-    }
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        w[2 * j] = acc[j].x;
-        w[2 * j + 1] = acc[j].y;
-    }
-    w[2 * K] = last;
-}
-
 // The taps of ND points (the two dimensions of one point, or one dimension).
 // The window is even, so taps m and -m share one pair of half-degree
-// polynomials in u = t^2,
+// polynomials in u = t^2 (coefficients read from kernel parameter space),
 //     w(t - m) = c0 + t (O + t E),   w(t + m) = c0 - t (O - t E),
 // and all share every coefficient read: for both dimensions 72 FMAs (64 of
 // them packed) and 32 constant reads a point at K = 6, where a Horner run per
@@ -285,68 +259,42 @@ __device__ __forceinline__ void weights_poly_d(float t, float (&w)[2 * K + 1], f
     dw[2 * K] = dlast;
 }
 
-// Derivative dw/dt of the same taps (d/dt of w(t - m)), closed form.
-//   interior: dw/du = w * (alpha s coth(alpha s) - 1) * (-u) / s^2
-//   edge:     dw/du = cn * g'(P) * (-2u),  g(P) = sinh(alpha sqrt(P))/sqrt(P),
-//             g' by its series near P = 0, closed forms elsewhere.
+// FP64 taps of both dimensions from the plan's polynomials (WinPoly64): taps
+// K - m and K + m share one pair of half-degree polynomials, and both
+// dimensions every coefficient read.
 template <int K>
-__device__ __forceinline__ void dweights_f32(float t, const float (&w)[2 * K + 1], float (&dw)[2 * K + 1],
-                                             float alpha, float cn) {
+__device__ __forceinline__ void weights_f64(double t1, double t2, double (&w1)[2 * K + 1], double (&w2)[2 * K + 1],
+                                            const WinPoly64 &P) {
+    const double ts[2] = {t1, t2}, us[2] = {t1 * t1, t2 * t2};
+    double *const ws[2] = {w1, w2};
 #pragma unroll
-    for (int a = 0; a <= 2 * K; ++a) {
-        const int m = a - K;
-        const float pa = static_cast<float>(K + m) - t;
-        const float pb = static_cast<float>(K - m) + t;
-        const float P = pa * pb;
-        const float u = t - static_cast<float>(m);
-        if (a != 0 && a != 2 * K) {
-            const float s = sqrtf(P);
-            const float as = alpha * s;
-            float coth = 1.0f;
-            if (K <= 3) {
-                const float e = __expf(-2.0f * as);
-                coth = (1.0f + e) / (1.0f - e);
+    for (int a = 0; a <= K; ++a) {
+        double e[2], o[2];
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            e[d] = P.e[kPoly64 - 1][a];
+            o[d] = P.o[kPoly64 - 1][a];
+        }
+#pragma unroll
+        for (int i = kPoly64 - 2; i >= 0; --i)
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+                if (i > 0 || a == K) e[d] = fma(e[d], us[d], P.e[i][a]);
+                if (a < K) o[d] = fma(o[d], us[d], P.o[i][a]);
             }
-            dw[a] = w[a] * (as * coth - 1.0f) * (-u) / P;
-        } else {
-            const float a2 = alpha * alpha;
-            float gp;
-            if (fabsf(a2 * P) < 0.5f) {
-                // alpha^3/6 + alpha^5 P/60 + alpha^7 P^2/1680 + alpha^9 P^3/90720
-                gp = alpha * a2 * (1.0f / 6.0f + a2 * P * (1.0f / 60.0f + a2 * P * (1.0f / 1680.0f + a2 * P * (1.0f / 90720.0f))));
-            } else if (P > 0.0f) {
-                const float s = sqrtf(P), as = alpha * s;
-                gp = (as * coshf(as) - sinhf(as)) / (2.0f * s * P);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            if (a == K) {
+                ws[d][K] = e[d];
             } else {
-                const float s = sqrtf(-P), as = alpha * s;
-                gp = -(as * cosf(as) - sinf(as)) / (2.0f * s * (-P));
+                ws[d][a] = fma(ts[d], fma(ts[d], e[d], o[d]), P.e[0][a]);
+                ws[d][2 * K - a] = fma(-ts[d], fma(-ts[d], e[d], o[d]), P.e[0][a]);
             }
-            dw[a] = cn * gp * (-2.0f * u);
         }
     }
 }
 
-// FP64 versions: the reference formula directly (FP64 plans are the
-// precision / compatibility path; GB300 FP64 throughput is low, so the FP32
-// plans never use these in their hot loops).
-template <int K>
-__device__ __forceinline__ void weights_f64(double t, double (&w)[2 * K + 1], double alpha, double cn) {
-#pragma unroll
-    for (int a = 0; a <= 2 * K; ++a) {
-        const int m = a - K;
-        const double pa = static_cast<double>(K + m) - t;
-        const double pb = static_cast<double>(K - m) + t;
-        const double P = pa * pb;
-        const double s = sqrt(fabs(P));
-        if (s == 0.0) {
-            w[a] = cn * alpha;
-        } else {
-            const double v = (P > 0.0) ? sinh(alpha * s) : sin(alpha * s);
-            w[a] = cn * v / s;
-        }
-    }
-}
-
+// Slopes of the FP64 taps, the reference formula's derivative directly.
 template <int K>
 __device__ __forceinline__ void dweights_f64(double t, double (&dw)[2 * K + 1], double alpha, double cn) {
 #pragma unroll

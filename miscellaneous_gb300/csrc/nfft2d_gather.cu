@@ -19,7 +19,7 @@
 // use k_gather_direct_f32 / k_grad_direct_f32 (two taps per 16-byte load,
 // bounded registers, compensated row sum in the gather), the gather of dense
 // sets and wide windows k_gather_tc (tc_gather_pays); FP64 plans the generic
-// k_gather_direct.
+// k_gather_direct_f64.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -35,6 +35,9 @@ namespace nfft2d {
 namespace {
 
 constexpr int kThreads = 256;
+// CTAs of the FP64 kernels: their time is FP64 arithmetic, which more and
+// smaller CTAs spread over the SMs more evenly.
+constexpr int kThreads64 = 64;
 
 template <int K>
 __device__ __forceinline__ void issue_patch(const CUtensorMap *map, const int4 *__restrict__ chunks, int c,
@@ -161,88 +164,60 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? 4 : 2) k_gather_tiled(co
     }
 }
 
-template <typename Real>
-struct CxOf;
-template <>
-struct CxOf<float> {
-    using type = float2;
-};
-template <>
-struct CxOf<double> {
-    using type = double2;
-};
-
-template <int K, typename Real>
-__device__ __forceinline__ void weights_any(Real t, Real (&w)[2 * K + 1], const KArgs &a) {
-    if constexpr (sizeof(Real) == 4)
-        weights_poly<K>(t, w, a.poly);
-    else
-        weights_f64<K>(t, w, a.alpha_d, a.cn_d);
-}
-
-// Slopes dw/dt of the taps; the FP32 path re-evaluates w with them (the
-// same Horner steps, so w is unchanged).
-template <int K, typename Real>
-__device__ __forceinline__ void dweights_any(Real t, Real (&w)[2 * K + 1], Real (&dw)[2 * K + 1], const KArgs &a) {
-    if constexpr (sizeof(Real) == 4)
-        weights_poly_d<K>(t, w, dw, a.poly);
-    else
-        dweights_f64<K>(t, dw, a.alpha_d, a.cn_d);
-}
-
-template <int K, typename Real, typename RecT, int MODE>
-__global__ void __launch_bounds__(kThreads) k_gather_direct(const typename CxOf<Real>::type *__restrict__ grid,
-                                                            const RecT *__restrict__ recs,
-                                                            typename CxOf<Real>::type *__restrict__ out,
-                                                            const typename CxOf<Real>::type *__restrict__ vin,
-                                                            Real *__restrict__ g1, Real *__restrict__ g2,
-                                                            const __grid_constant__ KArgs a) {
-    using Cx = typename CxOf<Real>::type;
+// FP64 plans: one thread per sorted point.  Bound by the FP64 pipe (0.53
+// TFMA/s on GB300: 600 FMAs a point at K = 6, 0.11 ms per 10^5 points); the
+// closed-form taps took it to 390 us per 10^5 points, the polynomials to 119
+// (125 in CTAs of 256: 2.6 an SM).
+template <int K, int MODE>
+__global__ void __launch_bounds__(kThreads64) k_gather_direct_f64(const double2 *__restrict__ grid,
+                                                                const Rec64 *__restrict__ recs,
+                                                                double2 *__restrict__ out,
+                                                                const double2 *__restrict__ vin,
+                                                                double *__restrict__ g1, double *__restrict__ g2,
+                                                                const __grid_constant__ KArgs a,
+                                                                const __grid_constant__ WinPoly64 wp) {
     constexpr int W = 2 * K + 1;
-    const int i = blockIdx.x * kThreads + threadIdx.x;
+    const int i = blockIdx.x * kThreads64 + threadIdx.x;
     if (i >= a.M) return;
-    const RecT r = recs[i];
+    const Rec64 r = recs[i];
     const int mu1 = static_cast<int>(static_cast<unsigned>(r.mu) >> 16), mu2 = r.mu & 0xFFFF;
     const Geom g = a.g;
     if (mu1 >= g.n1 || mu2 >= g.n2) {
         latch_error(a.status, kErrBounds);
         return;
     }
-    const Cx *base = grid + static_cast<size_t>(mu1 + g.H - K) * g.C + (mu2 + g.H - K);
-    Real w1[W], w2[W];
-    weights_any<K, Real>(static_cast<Real>(r.t1), w1, a);
-    weights_any<K, Real>(static_cast<Real>(r.t2), w2, a);
+    const double2 *base = grid + static_cast<size_t>(mu1 + g.H - K) * g.C + (mu2 + g.H - K);
+    double w1[W], w2[W];
+    weights_f64<K>(r.t1, r.t2, w1, w2, wp);
+    const int io = a.binned_io ? i : r.orig;
     if constexpr (MODE == 0) {
-        Real sx = 0, sy = 0;
+        double sx = 0, sy = 0;
 #pragma unroll
         for (int rr = 0; rr < W; ++rr) {
-            const Cx *row = base + static_cast<size_t>(rr) * g.C;
-            Real rx = 0, ry = 0;
+            const double2 *row = base + static_cast<size_t>(rr) * g.C;
+            double rx = 0, ry = 0;
 #pragma unroll
             for (int q = 0; q < W; ++q) {
-                const Cx v = __ldg(row + q);
+                const double2 v = __ldg(row + q);
                 rx += w2[q] * v.x;
                 ry += w2[q] * v.y;
             }
             sx += w1[rr] * rx;
             sy += w1[rr] * ry;
         }
-        Cx o;
-        o.x = sx;
-        o.y = sy;
-        out[a.binned_io ? i : r.orig] = o;
+        out[io] = make_double2(sx, sy);
     } else {
-        Real d1[W], d2[W];
-        dweights_any<K, Real>(static_cast<Real>(r.t1), w1, d1, a);
-        dweights_any<K, Real>(static_cast<Real>(r.t2), w2, d2, a);
-        Real ax = 0, ay = 0, bx = 0, by = 0;
+        double d1[W], d2[W];
+        dweights_f64<K>(r.t1, d1, a.alpha_d, a.cn_d);
+        dweights_f64<K>(r.t2, d2, a.alpha_d, a.cn_d);
+        double ax = 0, ay = 0, bx = 0, by = 0;
 #pragma unroll
         for (int rr = 0; rr < W; ++rr) {
-            const Cx *row = base + static_cast<size_t>(rr) * g.C;
-            Real rx = 0, ry = 0, qx = 0, qy = 0;
+            const double2 *row = base + static_cast<size_t>(rr) * g.C;
+            double rx = 0, ry = 0, qx = 0, qy = 0;
 #pragma unroll
             for (int q = 0; q < W; ++q) {
-                const Cx v = __ldg(row + q);
+                const double2 v = __ldg(row + q);
                 rx += w2[q] * v.x;
                 ry += w2[q] * v.y;
                 qx += d2[q] * v.x;
@@ -253,15 +228,9 @@ __global__ void __launch_bounds__(kThreads) k_gather_direct(const typename CxOf<
             bx += w1[rr] * qx;
             by += w1[rr] * qy;
         }
-        const int io = a.binned_io ? i : r.orig;
-        const Cx v = __ldg(&vin[io]);
-        if constexpr (sizeof(Real) == 4) {
-            g1[io] = a.ds1 * (v.x * ax + v.y * ay);
-            g2[io] = a.ds2 * (v.x * bx + v.y * by);
-        } else {
-            g1[io] = a.ds1_d * (v.x * ax + v.y * ay);
-            g2[io] = a.ds2_d * (v.x * bx + v.y * by);
-        }
+        const double2 v = __ldg(&vin[io]);
+        g1[io] = a.ds1_d * (v.x * ax + v.y * ay);
+        g2[io] = a.ds2_d * (v.x * bx + v.y * by);
     }
 }
 
@@ -401,9 +370,9 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
     const int blocks = static_cast<int>((p->M + kThreads - 1) / kThreads);
     if (blocks == 0) return cudaSuccess;
     if (p->precision == NFFT2D_F64) {
-        k_gather_direct<K, double, Rec64, MODE><<<blocks, kThreads, 0, p->stream>>>(
+        k_gather_direct_f64<K, MODE><<<static_cast<unsigned>((p->M + kThreads64 - 1) / kThreads64), kThreads64, 0, p->stream>>>(
             static_cast<const double2 *>(p->grid), static_cast<const Rec64 *>(p->recs), static_cast<double2 *>(f),
-            static_cast<const double2 *>(v), static_cast<double *>(g1), static_cast<double *>(g2), a);
+            static_cast<const double2 *>(v), static_cast<double *>(g1), static_cast<double *>(g2), a, p->poly64);
     } else if constexpr (MODE == 0) {
         if constexpr (K >= 6) {
             if (tc_gather_pays(K, p->g, p->M)) {

@@ -51,6 +51,18 @@ struct __align__(8) WinPoly {
 // error of the FP64 fit on a dense grid (negative on invalid arguments).
 double fit_window_poly(double sigma, int K, WinPoly *out);
 
+// The FP64 window the same way, by the window's symmetry: for m = K - a,
+// w(t -+ m) = e[0][a] + t (+-O + t E) with E = sum e[i][a] u^(i-1) over i >= 1,
+// O = sum o[i][a] u^i, u = t^2 (the centre tap a = K has no O).  Fitted at the
+// Chebyshev nodes of u in [0, 1/4]; the closed form, one sinh or sin, square
+// root and division a tap, cost 5 times the FP64 operations.
+constexpr int kPoly64 = 9;
+struct WinPoly64 {
+    double e[kPoly64][kMaxK + 1], o[kPoly64][kMaxK + 1];
+};
+// Returns the max abs difference from the closed form on a dense grid.
+double fit_window_poly64(double sigma, int K, WinPoly64 *out);
+
 // Window constants of one plan (both precisions are filled).
 struct WinConst {
     double alpha;   // (2 - 1/sigma) pi - 0.01  (NFFT1_2D.m:11, NFFT2_2D.cu:27)
@@ -105,6 +117,7 @@ struct nfft2d_plan_s {
     nfft2d::Geom g{};
     nfft2d::WinConst w{};
     nfft2d::WinPoly poly{};      // FP32 window polynomials
+    nfft2d::WinPoly64 poly64{};  // FP64 window polynomials (FP64 plans)
     int chunk = 256;
     int gather_variant = NFFT2D_VARIANT_TILED;
     bool gather_auto = true;     // FP32: pick the gather by bin density at set_points

@@ -110,32 +110,96 @@ double nfft2d::fit_window_poly(double sigma, int K, WinPoly *out) {
     return maxerr;
 }
 
+double nfft2d::fit_window_poly64(double sigma, int K, WinPoly64 *out) {
+    if (!out || K < kMinK || K > kMaxK || !(sigma >= 1.0) || !std::isfinite(sigma)) return -1.0;
+    const double pi = 3.141592653589793238462643383279502884;
+    const double alpha = (2.0 - 1.0 / sigma) * pi - 0.01;
+    const double cn = K / std::sinh(alpha * K), tail = 1.0 - std::exp(-2.0 * alpha * K);
+    // the normalised window; inside, the exponential's argument is formed
+    // without cancellation, so the error stays near 1e-16 of the peak
+    auto win = [&](double u) {
+        const double P = (K - u) * (K + u);
+        const double s = std::sqrt(std::fabs(P));
+        if (s == 0.0) return cn * alpha;
+        if (P < 0) return cn * std::sin(alpha * s) / s;
+        return K * std::exp(-alpha * u * u / (s + K)) * (1.0 - std::exp(-2.0 * alpha * s)) / (s * tail);
+    };
+    std::memset(out, 0, sizeof(*out));
+    constexpr int n = kPoly64;
+    double maxerr = 0.0;
+    for (int a = 0; a <= K; ++a) {
+        const int m = K - a;
+        for (int odd = 0; odd < (m ? 2 : 1); ++odd) {
+            // interpolation at the Chebyshev nodes of v = 4u in [0, 1]
+            double A[n][n + 1];
+            for (int i = 0; i < n; ++i) {
+                const double v = 0.5 * (1.0 + std::cos(pi * (i + 0.5) / n)), t = 0.5 * std::sqrt(v);
+                double pw = 1.0;
+                for (int j = 0; j < n; ++j) {
+                    A[i][j] = pw;
+                    pw *= v;
+                }
+                A[i][n] = odd ? (win(t + m) - win(t - m)) / (2.0 * t) : 0.5 * (win(t + m) + win(t - m));
+            }
+            for (int col = 0; col < n; ++col) {
+                int piv = col;
+                for (int r = col + 1; r < n; ++r)
+                    if (std::fabs(A[r][col]) > std::fabs(A[piv][col])) piv = r;
+                for (int j = 0; j <= n; ++j) std::swap(A[col][j], A[piv][j]);
+                for (int r = col + 1; r < n; ++r) {
+                    const double f = A[r][col] / A[col][col];
+                    for (int j = col; j <= n; ++j) A[r][j] -= f * A[col][j];
+                }
+            }
+            double (*const c)[kMaxK + 1] = odd ? out->o : out->e;
+            for (int i = n - 1; i >= 0; --i) {
+                double v = A[i][n];
+                for (int j = i + 1; j < n; ++j) v -= A[i][j] * c[j][a];
+                c[i][a] = v / A[i][i];
+            }
+            for (int i = 0; i < n; ++i) c[i][a] *= std::ldexp(1.0, 2 * i);  // powers of u
+        }
+        for (int q = 0; q <= 1000; ++q) {
+            const double t = -0.5 + q / 1000.0, u = t * t;
+            double e = 0.0, o = 0.0;
+            for (int i = n - 1; i >= 0; --i) {
+                e = e * u + out->e[i][a];
+                o = o * u + out->o[i][a];
+            }
+            maxerr = std::max(maxerr, std::fabs(e + t * o - win(t + m)));
+        }
+    }
+    return maxerr;
+}
+
 namespace {
 // The fitted window of every (sigma, K) a process has used: plans of the same
 // window (every regridding of an FFBP image, every transform of a batch)
 // share one fit instead of refitting on each plan creation.
+template <typename Poly>
 struct PolyCacheEntry {
     double sigma;
     int K;
     double err;
-    nfft2d::WinPoly poly;
+    Poly poly;
 };
 std::mutex g_poly_mu;
-std::vector<PolyCacheEntry> g_poly_cache;
 
-double cached_window_poly(double sigma, int K, nfft2d::WinPoly *out) {
+template <typename Poly>
+double cached_window_poly(double (*fit)(double, int, Poly *), double sigma, int K, Poly *out) {
+    static std::vector<PolyCacheEntry<Poly>> cache;
     {
         std::lock_guard<std::mutex> lock(g_poly_mu);
-        for (const auto &e : g_poly_cache)
+        for (const auto &e : cache)
             if (e.sigma == sigma && e.K == K) {
                 *out = e.poly;
                 return e.err;
             }
     }
-    const double err = nfft2d::fit_window_poly(sigma, K, out);
+    const double err = fit(sigma, K, out);
     if (err >= 0.0) {
         std::lock_guard<std::mutex> lock(g_poly_mu);
-        if (g_poly_cache.size() < 64) g_poly_cache.push_back({sigma, K, err, *out});
+        if (cache.size() < 64) cache.push_back({sigma, K, err, *out});
     }
     return err;
 }
@@ -1521,8 +1585,12 @@ int create_plan(nfft2d_plan_s **out, int N1, int N2, double sigma, int K, int pr
     p->w.alpha = alpha;
     p->w.cn = K / std::sinh(alpha * K);
     p->w.kp = K / (1.0 - std::exp(-2.0 * alpha * K));
-    const double poly_err = cached_window_poly(sigma, K, &p->poly);
+    const double poly_err = cached_window_poly(nfft2d::fit_window_poly, sigma, K, &p->poly);
     if (!(poly_err >= 0.0 && poly_err < 1e-8)) return fail(NFFT2D_ERR_INTERNAL);
+    if (precision == NFFT2D_F64) {
+        const double err = cached_window_poly(nfft2d::fit_window_poly64, sigma, K, &p->poly64);
+        if (!(err >= 0.0 && err < 1e-13)) return fail(NFFT2D_ERR_INTERNAL);
+    }
 
     const size_t rs = real_size(precision);
     cudaError_t e;
