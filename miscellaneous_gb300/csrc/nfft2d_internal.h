@@ -20,6 +20,11 @@ constexpr int kErrTimeout = 1;
 constexpr int kErrBounds = 2;
 constexpr int kErrNonfinite = 4;
 
+// d_status: [0] work items, [1] error bits, [2] the spread's work counter, [3]
+// its own work items, [4] [5] the grid barrier of the one-launch transforms
+// (zero between launches).
+constexpr int kStatusWords = 6, kBarrierWord = 4;
+
 // One binned point, FP32 plans: fractional offsets t = sigma*x_grid - mu in
 // [-1/2, 1/2], packed wrapped cell (mu1 << 16 | mu2) and the caller's index.
 struct __align__(16) Rec32 {
@@ -134,7 +139,7 @@ struct nfft2d_plan_s {
     bool grid_external = false;  // grid owned by a batch (no free, no own cuFFT plan)
     void *deap1 = nullptr;       // N1 reals: S / phi(xi_k1), plan precision
     void *deap2 = nullptr;       // N2 reals
-    int *d_status = nullptr;     // [0] n_chunks, [1] error bits
+    int *d_status = nullptr;     // kStatusWords: [0] n_chunks, [1] error bits, see kBarrierWord
     int *h_status = nullptr;     // page-locked host copy of d_status
     unsigned *cell_count = nullptr;  // ncells + 1 counters / starts
     size_t ncells = 0;
@@ -170,6 +175,7 @@ struct nfft2d_plan_s {
     bool pruned_ok = false;
     int fft_mode = -1;                       // -1 auto, 0 2D plan, 1 pruned passes, 2 fused passes
     bool fused_ok = false;                   // twiddle tables of the fused passes are set up
+    bool small_ok = false;                   // the one-launch transforms fit the plan and the device
     float2 *tw1 = nullptr, *tw2 = nullptr;   // exp(-2 pi i m / n1), exp(-2 pi i m / n2)
     CUtensorMap tmap;  // 64-byte aligned by its own declaration
     CUtensorMap tmap_spread;  // box of one strip patch of the FP32 tiled spread
@@ -298,6 +304,12 @@ cudaError_t fused_type2_cols(const nfft2d_plan_s *p, int sign, const void *F);
 cudaError_t fused_type2_rows(const nfft2d_plan_s *p, int sign);
 cudaError_t fused_type1_rows(const nfft2d_plan_s *p, int sign);
 cudaError_t fused_type1_cols(const nfft2d_plan_s *p, int sign, void *F);
+
+// Whole transforms in one launch (nfft2d_small.cu): whether the plan's sizes
+// and the device take them, and the launches (points set).
+bool small_available(const nfft2d_plan_s *p);
+cudaError_t launch_small_type2(const nfft2d_plan_s *p, int sign, const void *F, void *f);
+cudaError_t launch_small_type1(const nfft2d_plan_s *p, int sign, const void *f, void *F);
 
 // One thread waits on an mbarrier phase that nothing completes, gives up
 // after `limit` polls and latches kErrTimeout in status[1] (the self-tests of

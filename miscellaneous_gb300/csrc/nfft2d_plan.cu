@@ -366,6 +366,26 @@ bool use_fused(const nfft2d_plan_s *p) {
     return p->fft_mode < 0 && 1LL * p->g.n1 * p->g.n2 < 2048LL * 2048LL;
 }
 
+// Whole transforms in one launch (nfft2d_small.cu) for small sets on small
+// grids, where launches and latency are most of the time: with the plan's own
+// choice of stages, and no stage to time.  Measured on GB300, one launch
+// against the separate kernels, w 6, us (forward | adjoint):
+//    64^2 coefficients   4096 points  15.2 / 19.6 | 16.5 / 34.9
+//    64^2               16000         19.6 / 21.6 | 24.8 / 44.6
+//   128^2                4096         18.5 / 20.5 | 22.6 / 32.5
+//   128^2               16000         20.6 / 20.6 | 28.7 / 37.1
+//   128^2               30000         24.6 / 22.6 | 34.5 / 39.1
+//   256^2                8000         30.8 / 22.6 | 38.0 / 35.1
+// so up to 256^2 cells, with 2^13 points forward (2^14 on 128^2 cells) and
+// 2^15 points adjoint.
+bool use_small(const nfft2d_plan_s *p, bool adjoint) {
+    if (!p->small_ok || !p->gather_auto || p->spread_variant != NFFT2D_VARIANT_TILED || p->fft_mode >= 0 ||
+        p->timer.on || p->g.T != 16 || p->g.SW != spread_strip_width(p->K) || p->chunk > kSpreadItemMax)
+        return false;
+    const long long cells = 1LL * p->g.n1 * p->g.n2;
+    return cells <= 256 * 256 && p->M <= (adjoint ? 1 << 15 : cells <= 128 * 128 ? 1 << 14 : 1 << 13);
+}
+
 // The automatic FP32 gather: the direct 16-byte-load gather from 128 points
 // per 16 x 16 tile or 2^18 points up, the TMA-tiled patches for small, thin
 // point sets.  Measured on GB300: tiled for 4096 points on 64^2
@@ -1221,8 +1241,11 @@ int setup_grid(nfft2d_plan_s *p) {
         const int sf = ensure_ffts(p);
         if (sf != NFFT2D_OK) return sf;
     }
-    if (p->precision == NFFT2D_F32) return make_tensor_map(p);
-    return NFFT2D_OK;
+    p->small_ok = false;
+    if (p->precision != NFFT2D_F32) return NFFT2D_OK;
+    const int st = make_tensor_map(p);
+    if (st == NFFT2D_OK) p->small_ok = small_available(p);
+    return st;
 }
 
 // (Re)allocate the bin counters for the current tile geometry.
@@ -1598,10 +1621,10 @@ int create_plan(nfft2d_plan_s **out, int N1, int N2, double sigma, int K, int pr
     if ((st = setup_bins(p)) != NFFT2D_OK) return fail(st);
     if ((e = plan_malloc(reinterpret_cast<void **>(&p->deap1), rs * N1)) != cudaSuccess) return fail(status_from_cuda(e));
     if ((e = plan_malloc(reinterpret_cast<void **>(&p->deap2), rs * N2)) != cudaSuccess) return fail(status_from_cuda(e));
-    if ((e = plan_malloc(reinterpret_cast<void **>(&p->d_status), 4 * sizeof(int))) != cudaSuccess) return fail(status_from_cuda(e));
+    if ((e = plan_malloc(reinterpret_cast<void **>(&p->d_status), kStatusWords * sizeof(int))) != cudaSuccess) return fail(status_from_cuda(e));
     if ((e = plan_malloc_host(reinterpret_cast<void **>(&p->h_status), 4 * sizeof(int))) != cudaSuccess)
         return fail(status_from_cuda(e));
-    if ((e = cudaMemsetAsync(p->d_status, 0, 4 * sizeof(int), p->stream)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(p->d_status, 0, kStatusWords * sizeof(int), p->stream)) != cudaSuccess)
         return fail(status_from_cuda(e));
 
     // Deapodization tables S / phi(xi_k), S = sinh(alpha K)/(pi K) (the
@@ -2036,6 +2059,10 @@ static int nfft2d_type2_impl(nfft2d_plan p, int sign, const void *F, void *f) {
     if (!F || (p->M > 0 && !f)) return NFFT2D_ERR_INVALID_ARG;
     timer_reset(p, CALL_TYPE2);
     if (p->M == 0) return NFFT2D_OK;
+    if (use_small(p, false)) {
+        NFFT_TRY_CUDA(launch_small_type2(p, sign, F, f));
+        return NFFT2D_OK;
+    }
     int st = type2_prepare(p, sign, F);
     if (st != NFFT2D_OK) return st;
     stage_begin(p, ST_GATHER);
@@ -2053,6 +2080,10 @@ static int nfft2d_type1_impl(nfft2d_plan p, int sign, const void *f, void *F) {
     const Geom &g = p->g;
     if (p->M == 0) {
         NFFT_TRY_CUDA(cudaMemsetAsync(F, 0, cplx_size(p->precision) * p->N1 * p->N2, p->stream));
+        return NFFT2D_OK;
+    }
+    if (use_small(p, true)) {
+        NFFT_TRY_CUDA(launch_small_type1(p, sign, f, F));
         return NFFT2D_OK;
     }
     stage_begin(p, ST_SPREAD);
@@ -2149,6 +2180,15 @@ int nfft2d_bin_and_forward(nfft2d_plan p, long long M, const void *x1, const voi
         }
     };
     const void *Fd = F;
+    if (M > 0 && use_small(p, false)) {  // one launch after the binning: nothing left to overlap
+        if (F_host) {
+            NFFT_TRY_CUDA(cudaMemcpyAsync(p->F_stage, F, F_bytes, cudaMemcpyHostToDevice, main));
+            if (user_ev) NFFT_TRY_CUDA(cudaEventRecord(user_ev, main));
+            Fd = p->F_stage;
+        }
+        NFFT_TRY_CUDA(launch_small_type2(p, -1, Fd, f));
+        return NFFT2D_OK;
+    }
     if (F_host) {
         NFFT_TRY_CUDA(cudaStreamWaitEvent(p->aux, coords_read, 0));
         NFFT_TRY_CUDA(cudaMemcpyAsync(p->F_stage, F, F_bytes, cudaMemcpyHostToDevice, p->aux));
@@ -2230,7 +2270,10 @@ int nfft2d::apply_status(nfft2d_plan_s *p) {
     // they are read (the stream is idle here)
     const int bits = hs[1];
     if (bits) NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status + 1, 0, sizeof(int), p->stream));
-    if (bits & kErrTimeout) return NFFT2D_ERR_DEVICE_TIMEOUT;
+    if (bits & kErrTimeout) {  // a grid barrier that was given up on leaves its words behind
+        NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status + kBarrierWord, 0, 2 * sizeof(int), p->stream));
+        return NFFT2D_ERR_DEVICE_TIMEOUT;
+    }
     if (bits & kErrBounds) return NFFT2D_ERR_DEVICE_BOUNDS;
     return NFFT2D_OK;
 }
