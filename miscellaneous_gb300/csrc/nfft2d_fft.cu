@@ -267,20 +267,27 @@ __global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_cols_pad(const flo
     prefetch_twiddles<true>(tws, a.logn1, a.logP, a.s, tw);
     const int P = 1 << a.logP, n1 = a.n1;
     const int bc0 = blockIdx.x << a.logP;
-    // every thread owns 16 elements (blockDim = P n / 16): all loads first
+    // every thread owns 16 elements (blockDim = P n / 16) of one column
+    // (blockDim is a multiple of P): all loads first, rows outside the band
+    // loading the band's edge and zeroed after -- a load behind a branch is
+    // waited for there (1024^2: 7.4 -> 6.8 us)
+    const int bc_in = bc0 + (threadIdx.x & (P - 1)), j_in = band_coef(min(bc_in, a.N2 - 1), a.N2);
+    const float s2 = __ldg(d2 + j_in);
     float2 v[16];
+    float s1[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
-        const int e = threadIdx.x + u * blockDim.x;
-        const int q = e & (P - 1), r = e >> a.logP, bc = bc0 + q;
-        v[u] = make_float2(0.f, 0.f);
-        const int k1 = r < n1 / 2 ? r : r - n1;
-        if (bc < a.N2 && k1 >= -a.N1 / 2 && k1 < a.N1 / 2) {
-            const int i = k1 + a.N1 / 2, j = band_coef(bc, a.N2);
-            const float sc = __ldg(d1 + i) * __ldg(d2 + j);
-            const float2 f = __ldg(F + static_cast<size_t>(i) * a.N2 + j);
-            v[u] = make_float2(f.x * sc, f.y * sc);
-        }
+        const int r = (threadIdx.x + u * blockDim.x) >> a.logP, k1 = r < n1 / 2 ? r : r - n1;
+        const int i = min(max(k1 + a.N1 / 2, 0), a.N1 - 1);
+        s1[u] = __ldg(d1 + i);
+        v[u] = __ldg(F + static_cast<size_t>(i) * a.N2 + j_in);
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int r = (threadIdx.x + u * blockDim.x) >> a.logP, k1 = r < n1 / 2 ? r : r - n1;
+        const float sc = s1[u] * s2;
+        const bool band = bc_in < a.N2 && k1 >= -a.N1 / 2 && k1 < a.N1 / 2;
+        v[u] = band ? make_float2(v[u].x * sc, v[u].y * sc) : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < 16; ++u) fsm[pad16(threadIdx.x + u * blockDim.x)] = v[u];
