@@ -91,6 +91,45 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 __device__ __forceinline__ void latch_error(int *status, int bit) { atomicOr(status + 1, bit); }
 
 // ---------------------------------------------------------------------------
+// barrier of a cooperative grid of kGridCtas CTAs (all resident: one an SM)
+// ---------------------------------------------------------------------------
+constexpr int kGridCtas = 128;
+// What any CTA wrote before it arrived, every thread of the kernel sees after
+// the wait; `target`: the CTAs' arrivals so far.  False, latched, if the wait
+// runs out (the CTA leaves; so do the others, by their own waits).
+__device__ __forceinline__ void grid_arrive(int *status) {
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(status + kBarrierWord) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(int *status, int target) {
+    __shared__ int ok;
+    if (threadIdx.x == 0) {
+        int seen = 0;
+        uint32_t spins = 0;
+        do
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(status + kBarrierWord) : "memory");
+        while (seen < target && ++spins < kSpinLimit);
+        ok = seen >= target;
+        if (!ok) latch_error(status, kErrTimeout);
+    }
+    __syncthreads();
+    return ok != 0;
+}
+__device__ __forceinline__ bool grid_barrier(int *status, int target) {
+    grid_arrive(status);
+    return grid_wait(status, target);
+}
+// The last CTA to come here leaves the barrier's words zero for the next launch.
+__device__ __forceinline__ void grid_done(int *status) {
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(status + kBarrierWord + 1, 1) == kGridCtas - 1) {
+        status[kBarrierWord] = 0;
+        status[kBarrierWord + 1] = 0;
+    }
+}
+
+
+// ---------------------------------------------------------------------------
 // Window pair.  The reference window (NFFT1_2D.m:34-36, NFFT2_2D.cu:112-122)
 //     phi_hat(u) = (1/pi) sinh(alpha s)/s,  s = sqrt(K^2 - u^2)
 // (sin form for |u| > K) is used here normalised to 1 at u = 0:

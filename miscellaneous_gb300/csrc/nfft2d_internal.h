@@ -144,7 +144,7 @@ struct nfft2d_plan_s {
     unsigned *cell_count = nullptr;  // ncells + 1 counters / starts
     size_t ncells = 0;
     unsigned *scan_tmp = nullptr;
-    size_t scan_tmp_elems = 0;
+    size_t scan_tmp_elems = 0, tile_count_at = 0;
 
     // points
     long long M = 0;             // points set (0: none)

@@ -796,6 +796,149 @@ __global__ void k_bin_gather(const RecT *__restrict__ tmp, const int *__restrict
 }
 
 // ---------------------------------------------------------------------------
+// Binning of one small point set in one cooperative launch: the passes above
+// with grid barriers for launch boundaries.  The points stay in their threads'
+// registers from the reduction to their sorted place, and the per-tile counts
+// that place cells and work items are added up beside the cells' own.  Bound
+// by three barriers (1.5 us each) and a round trip to L2 per phase; as two
+// fills and five launches it was bound by the launches.  The counts that the
+// host needs are written to page-locked memory, not copied there.  set_points
+// with its read-back, 4096 points on 128^2 cells: 41 -> 23 us.
+// ---------------------------------------------------------------------------
+constexpr int kOneBinThreads = 512, kOneBinItems = 2;
+constexpr long long kOneBinPoints = 1LL * kGridCtas * kOneBinThreads * kOneBinItems;
+constexpr int kOneBinTiles = 2048;
+
+struct OneBinArgs {
+    const void *x1, *x2;
+    int M;
+    double o1, o2, s1, s2;  // as k_bin_pass1
+    float s1f, s2f;
+    int exact;
+    Geom g;
+    void *recs;
+    int *src;
+    unsigned *cell_count, *tile_count;
+    int4 *chunks;
+    int chunk;
+    int *status;
+    int *host;  // page-locked copy of status[0], status[1], or null
+};
+
+template <typename CT, typename RecT>
+__global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_constant__ OneBinArgs a) {
+    constexpr int kStride = kGridCtas * kOneBinThreads, kWarps = kOneBinThreads / 32;
+    __shared__ unsigned tile_start[kOneBinTiles], item_start[kOneBinTiles];
+    __shared__ unsigned long long warp_tot[kWarps];
+    const Geom &g = a.g;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, gid = blockIdx.x * kOneBinThreads + tid;
+    const int ntiles = g.tiles1 * g.tiles2, cpt = g.T * g.T, ncells = ntiles * cpt;
+    for (int i = gid; i < ncells; i += kStride) a.cell_count[i] = 0u;
+    if (gid < ntiles) a.tile_count[gid] = 0u;
+    if (gid < 4) a.status[gid] = 0;
+    grid_arrive(a.status);
+    RecT r[kOneBinItems];
+    unsigned key[kOneBinItems], rank[kOneBinItems];
+    bool bad = false;
+#pragma unroll
+    for (int u = 0; u < kOneBinItems; ++u) {
+        const int i = min(gid + u * kStride, a.M - 1);
+        int mu1, mu2;
+        const bool ok1 = reduce_coord(__ldg(static_cast<const CT *>(a.x1) + i), a.o1, a.s1, a.s1f, a.exact != 0, g.n1,
+                                      mu1, r[u].t1);
+        const bool ok2 = reduce_coord(__ldg(static_cast<const CT *>(a.x2) + i), a.o2, a.s2, a.s2f, a.exact != 0, g.n2,
+                                      mu2, r[u].t2);
+        if (!ok1 || !ok2) {  // as k_bin_pass1: reported, and binned at cell 0 with t = 0
+            bad = true;
+            mu1 = mu2 = 0;
+            r[u].t1 = r[u].t2 = 0;
+        }
+        key[u] = cell_key(g, mu1, mu2);
+        r[u].mu = (mu1 << 16) | mu2;
+        r[u].orig = i;
+    }
+    if (!grid_wait(a.status, kGridCtas)) return;  // the counters are zero
+    if (bad) latch_error(a.status, kErrNonfinite);
+#pragma unroll
+    for (int u = 0; u < kOneBinItems; ++u) {
+        const bool have = gid + u * kStride < a.M;
+        if (have) rank[u] = atomicAdd(a.cell_count + key[u], 1u);
+        // one addition per tile and warp: the points of a dense set share it
+        const unsigned t = have ? key[u] / cpt : 0xffffffffu, same = __match_any_sync(0xffffffffu, t);
+        if (have && lane == __ffs(same) - 1) atomicAdd(a.tile_count + t, static_cast<unsigned>(__popc(same)));
+    }
+    if (!grid_barrier(a.status, 2 * kGridCtas)) return;
+    // where every tile's points and work items start, in each CTA: (points,
+    // items) scanned as one 64-bit word
+    unsigned long long before = 0;
+    for (int t0 = 0; t0 < ntiles; t0 += kOneBinThreads) {
+        const int t = t0 + tid;
+        const unsigned n = t < ntiles ? __ldcg(a.tile_count + t) : 0u;
+        const unsigned long long v = static_cast<unsigned long long>(n) << 32 | (n + a.chunk - 1) / a.chunk;
+        unsigned long long incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) warp_tot[wid] = incl;
+        __syncthreads();
+        unsigned long long excl = before + incl - v;
+        for (int w = 0; w < kWarps; ++w) {
+            const unsigned long long y = warp_tot[w];
+            if (w < wid) excl += y;
+            before += y;
+        }
+        if (t < ntiles) {
+            tile_start[t] = static_cast<unsigned>(excl >> 32);
+            item_start[t] = static_cast<unsigned>(excl);
+        }
+        __syncthreads();
+    }
+    if (gid == 0) {
+        const int items = static_cast<int>(static_cast<unsigned>(before));
+        a.cell_count[ncells] = static_cast<unsigned>(a.M);
+        a.status[0] = items;
+        if (a.host) {
+            a.host[1] = __ldcg(a.status + 1);
+            a.host[0] = items;
+        }
+    }
+    // a warp per tile: the starts of its cells, its work items
+    for (int t = wid * kGridCtas + blockIdx.x; t < ntiles; t += kWarps * kGridCtas) {
+        unsigned *cells = a.cell_count + static_cast<size_t>(t) * cpt;
+        unsigned start = tile_start[t];
+#pragma unroll 4
+        for (int c0 = 0; c0 < cpt; c0 += 32) {
+            const unsigned n = c0 + lane < cpt ? __ldcg(cells + c0 + lane) : 0u;
+            unsigned incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (c0 + lane < cpt) cells[c0 + lane] = start + incl - n;
+            start += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        const unsigned count = start - tile_start[t];
+        for (unsigned c = lane; c * a.chunk < count; c += 32)
+            a.chunks[item_start[t] + c] =
+                make_int4(t, static_cast<int>(tile_start[t] + c * a.chunk),
+                          static_cast<int>(min(count - c * a.chunk, static_cast<unsigned>(a.chunk))), 0);
+    }
+    if (!grid_barrier(a.status, 3 * kGridCtas)) return;
+#pragma unroll
+    for (int u = 0; u < kOneBinItems; ++u) {
+        const int i = gid + u * kStride;
+        if (i >= a.M) continue;
+        const unsigned q = __ldcg(a.cell_count + key[u]) + rank[u];
+        static_cast<RecT *>(a.recs)[q] = r[u];
+        a.src[q] = i;
+    }
+    grid_done(a.status);
+}
+
+// ---------------------------------------------------------------------------
 // Binning of many small point sets at once (the transforms of a batch): one
 // 1024-thread CTA per transform does the whole counting sort with its cell
 // counters in shared memory -- reduction, key and rank (shared atomics),
@@ -1261,6 +1404,8 @@ int setup_bins(nfft2d_plan_s *p) {
     // 64-bit state words of three scans: cells, work items, the spread's own items
     p->scan_tmp_elems = 2 * (scan_state_words(p->ncells + 1, kCellScanThreads * kCellScanItems) +
                              2 * scan_state_words(ntiles + 1, kItemScanThreads * kItemScanItems));
+    p->tile_count_at = p->scan_tmp_elems;  // then a counter per tile (k_bin_one)
+    p->scan_tmp_elems += ntiles;
     NFFT_TRY_CUDA(plan_malloc(reinterpret_cast<void **>(&p->cell_count), sizeof(unsigned) * (p->ncells + 1)));
     NFFT_TRY_CUDA(plan_malloc(reinterpret_cast<void **>(&p->scan_tmp), sizeof(unsigned) * p->scan_tmp_elems));
     return NFFT2D_OK;
@@ -1906,6 +2051,35 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
     return status;
 }
 
+// One launch bins sets of up to 2^17 points (two a thread) on up to 2048 tiles.
+// Measured on GB300, set_points with its read-back, us, separate passes -> one
+// launch: 4096 points on 128^2 cells 41 -> 23; 16000 on 256^2 47 -> 26; 130000
+// on 512^2 49 -> 36 (all in one patch of the grid: 52 -> 39); FP64 130000 on
+// 512^2 50 -> 39.  A binning that runs beside the padding and the FFT
+// (`overlapped`) has its grid wait for their CTAs: 43 -> 28 at 4096 points, 51
+// -> 45 at 65000, but 47 -> 48 at 130000, and in FP64, whose FFT is cuFFT's,
+// 74 -> 89 and 267 -> 281; so FP32 and 2^16 points there.
+static bool use_one_bin(const nfft2d_plan_s *p, long long M, bool overlapped) {
+    return M <= kOneBinPoints && (!overlapped || (p->precision == NFFT2D_F32 && M <= kOneBinPoints / 2)) &&
+           1LL * p->g.tiles1 * p->g.tiles2 <= kOneBinTiles && p->chunk <= kSpreadItemMax && p->num_sms >= kGridCtas;
+}
+
+static cudaError_t launch_one_bin(const nfft2d_plan_s *p, int coord_dtype, const OneBinArgs &a) {
+    const bool f64 = p->precision == NFFT2D_F64;
+    auto kernel = coord_dtype == NFFT2D_COORD_F64 ? (f64 ? k_bin_one<double, Rec64> : k_bin_one<double, Rec32>)
+                                                  : (f64 ? k_bin_one<float, Rec64> : k_bin_one<float, Rec32>);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kGridCtas);
+    cfg.blockDim = dim3(kOneBinThreads);
+    cfg.stream = p->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, const void *x2, int coord_dtype,
                               double u1, double u2, double o1, double o2, bool async, cudaEvent_t coords_read) {
     if (!p) return NFFT2D_ERR_INVALID_ARG;
@@ -1942,68 +2116,84 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
     const int exact = (coord_dtype == NFFT2D_COORD_F32 && pow2 && o1 == 0.0 && o2 == 0.0) ? 1 : 0;
     const float s1f = static_cast<float>(s1), s2f = static_cast<float>(s2);
     stage_begin(p, ST_SORT);
-    NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status, 0, 4 * sizeof(int), p->stream));
-    NFFT_TRY_CUDA(cudaMemsetAsync(p->cell_count, 0, sizeof(unsigned) * (p->ncells + 1), p->stream));
-    const int Mi = static_cast<int>(M);
-    const int blocks = (Mi + 255) / 256;
-    // ticket + tile words of the cell scan, then of the work-item scan
-    unsigned long long *scan_state = reinterpret_cast<unsigned long long *>(p->scan_tmp);
-    constexpr int kCellTile = kCellScanThreads * kCellScanItems, kItemTile = kItemScanThreads * kItemScanItems;
-    const size_t item_words = scan_state_words(static_cast<size_t>(g.tiles1) * g.tiles2 + 1, kItemTile);
-    const int scan_words = static_cast<int>(scan_state_words(p->ncells + 1, kCellTile) + 2 * item_words);
-    // the binning's arrays against L2: coordinates, tmp records, keys and
-    // ranks, the inverse permutation, sorted records, cell counters
-    const size_t rec_bytes = p->precision == NFFT2D_F64 ? sizeof(Rec64) : sizeof(Rec32);
-    const size_t bin_bytes = static_cast<size_t>(M) * ((coord_dtype == NFFT2D_COORD_F64 ? 16 : 8) + 2 * rec_bytes + 12) +
-                             4 * (p->ncells + 1);
-    const bool stream = bin_bytes > static_cast<size_t>(p->l2_bytes);
-    auto bin = [&](auto ct, auto rt, auto st) -> cudaError_t {
-        using CT = decltype(ct);
-        using RecT = decltype(rt);
-        constexpr bool S = decltype(st)::value;
-        k_bin_pass1<CT, RecT, S><<<blocks, 256, 0, p->stream>>>(
-            static_cast<const CT *>(x1), static_cast<const CT *>(x2), Mi, o1, o2, s1, s2, s1f, s2f, exact, g,
-            static_cast<RecT *>(p->tmp_recs), p->keyrank, p->cell_count, p->d_status, scan_state, scan_words);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        if (coords_read && (e = cudaEventRecord(coords_read, p->stream)) != cudaSuccess) return e;  // coordinates read
-        const size_t cells_n = p->ncells + 1;
-        k_scan_counts<<<static_cast<unsigned>((cells_n + kCellTile - 1) / kCellTile), kCellScanThreads, 0,
-                        p->stream>>>(p->cell_count, cells_n, scan_state, p->d_status);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_bin_invert<S><<<blocks, 256, 0, p->stream>>>(p->keyrank, p->cell_count, Mi, p->src);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_bin_gather<RecT, S><<<blocks, 256, 0, p->stream>>>(static_cast<const RecT *>(p->tmp_recs), p->src, Mi,
-                                                              static_cast<RecT *>(p->recs));
-        return cudaGetLastError();
-    };
-    using Yes = std::true_type;
-    using No = std::false_type;
-    cudaError_t be;
-    if (p->precision == NFFT2D_F64) {
-        if (coord_dtype == NFFT2D_COORD_F64)
-            be = stream ? bin(double{}, Rec64{}, Yes{}) : bin(double{}, Rec64{}, No{});
-        else
-            be = stream ? bin(float{}, Rec64{}, Yes{}) : bin(float{}, Rec64{}, No{});
+    const int *hs = p->h_status;  // page-locked
+    const bool one = use_one_bin(p, M, coords_read != nullptr);
+    if (one) {
+        OneBinArgs a{};
+        a.x1 = x1, a.x2 = x2, a.M = static_cast<int>(M);
+        a.o1 = o1, a.o2 = o2, a.s1 = s1, a.s2 = s2, a.s1f = s1f, a.s2f = s2f, a.exact = exact;
+        a.g = g;
+        a.recs = p->recs, a.src = p->src, a.cell_count = p->cell_count, a.tile_count = p->scan_tmp + p->tile_count_at;
+        a.chunks = p->chunks, a.chunk = p->chunk;
+        a.status = p->d_status;
+        a.host = async ? nullptr : p->h_status;
+        if (!async) p->h_status[0] = -1;  // until the kernel has the counts
+        NFFT_TRY_CUDA(launch_one_bin(p, coord_dtype, a));
+        if (coords_read) NFFT_TRY_CUDA(cudaEventRecord(coords_read, p->stream));
     } else {
-        if (coord_dtype == NFFT2D_COORD_F64)
-            be = stream ? bin(double{}, Rec32{}, Yes{}) : bin(double{}, Rec32{}, No{});
-        else
-            be = stream ? bin(float{}, Rec32{}, Yes{}) : bin(float{}, Rec32{}, No{});
-    }
-    NFFT_TRY_CUDA(be);
-    const size_t cells_n = p->ncells + 1;
-    const int ntiles = g.tiles1 * g.tiles2;
-    const unsigned emit_blocks = static_cast<unsigned>((ntiles + 1 + kItemTile - 1) / kItemTile);
-    unsigned long long *item_state = scan_state + scan_state_words(cells_n, kCellTile);
-    k_scan_emit_chunks<<<emit_blocks, kItemScanThreads, 0, p->stream>>>(
-        p->cell_count, ntiles, g.T * g.T, p->chunk, p->chunks, item_state, p->d_status, p->d_status);
-    NFFT_TRY_CUDA(cudaGetLastError());
-    if (p->chunk > kSpreadItemMax) {  // the spread's own work list, count in status[3]
+        NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status, 0, 4 * sizeof(int), p->stream));
+        NFFT_TRY_CUDA(cudaMemsetAsync(p->cell_count, 0, sizeof(unsigned) * (p->ncells + 1), p->stream));
+        const int Mi = static_cast<int>(M);
+        const int blocks = (Mi + 255) / 256;
+        // ticket + tile words of the cell scan, then of the work-item scan
+        unsigned long long *scan_state = reinterpret_cast<unsigned long long *>(p->scan_tmp);
+        constexpr int kCellTile = kCellScanThreads * kCellScanItems, kItemTile = kItemScanThreads * kItemScanItems;
+        const size_t item_words = scan_state_words(static_cast<size_t>(g.tiles1) * g.tiles2 + 1, kItemTile);
+        const int scan_words = static_cast<int>(scan_state_words(p->ncells + 1, kCellTile) + 2 * item_words);
+        // the binning's arrays against L2: coordinates, tmp records, keys and
+        // ranks, the inverse permutation, sorted records, cell counters
+        const size_t rec_bytes = p->precision == NFFT2D_F64 ? sizeof(Rec64) : sizeof(Rec32);
+        const size_t bin_bytes = static_cast<size_t>(M) * ((coord_dtype == NFFT2D_COORD_F64 ? 16 : 8) + 2 * rec_bytes + 12) +
+                                 4 * (p->ncells + 1);
+        const bool stream = bin_bytes > static_cast<size_t>(p->l2_bytes);
+        auto bin = [&](auto ct, auto rt, auto st) -> cudaError_t {
+            using CT = decltype(ct);
+            using RecT = decltype(rt);
+            constexpr bool S = decltype(st)::value;
+            k_bin_pass1<CT, RecT, S><<<blocks, 256, 0, p->stream>>>(
+                static_cast<const CT *>(x1), static_cast<const CT *>(x2), Mi, o1, o2, s1, s2, s1f, s2f, exact, g,
+                static_cast<RecT *>(p->tmp_recs), p->keyrank, p->cell_count, p->d_status, scan_state, scan_words);
+            cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+            if (coords_read && (e = cudaEventRecord(coords_read, p->stream)) != cudaSuccess) return e;  // coordinates read
+            const size_t cells_n = p->ncells + 1;
+            k_scan_counts<<<static_cast<unsigned>((cells_n + kCellTile - 1) / kCellTile), kCellScanThreads, 0,
+                            p->stream>>>(p->cell_count, cells_n, scan_state, p->d_status);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            k_bin_invert<S><<<blocks, 256, 0, p->stream>>>(p->keyrank, p->cell_count, Mi, p->src);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            k_bin_gather<RecT, S><<<blocks, 256, 0, p->stream>>>(static_cast<const RecT *>(p->tmp_recs), p->src, Mi,
+                                                                  static_cast<RecT *>(p->recs));
+            return cudaGetLastError();
+        };
+        using Yes = std::true_type;
+        using No = std::false_type;
+        cudaError_t be;
+        if (p->precision == NFFT2D_F64) {
+            if (coord_dtype == NFFT2D_COORD_F64)
+                be = stream ? bin(double{}, Rec64{}, Yes{}) : bin(double{}, Rec64{}, No{});
+            else
+                be = stream ? bin(float{}, Rec64{}, Yes{}) : bin(float{}, Rec64{}, No{});
+        } else {
+            if (coord_dtype == NFFT2D_COORD_F64)
+                be = stream ? bin(double{}, Rec32{}, Yes{}) : bin(double{}, Rec32{}, No{});
+            else
+                be = stream ? bin(float{}, Rec32{}, Yes{}) : bin(float{}, Rec32{}, No{});
+        }
+        NFFT_TRY_CUDA(be);
+        const size_t cells_n = p->ncells + 1;
+        const int ntiles = g.tiles1 * g.tiles2;
+        const unsigned emit_blocks = static_cast<unsigned>((ntiles + 1 + kItemTile - 1) / kItemTile);
+        unsigned long long *item_state = scan_state + scan_state_words(cells_n, kCellTile);
         k_scan_emit_chunks<<<emit_blocks, kItemScanThreads, 0, p->stream>>>(
-            p->cell_count, ntiles, g.T * g.T, kSpreadItemMax, p->items, item_state + item_words, p->d_status,
-            p->d_status + 3);
+            p->cell_count, ntiles, g.T * g.T, p->chunk, p->chunks, item_state, p->d_status, p->d_status);
         NFFT_TRY_CUDA(cudaGetLastError());
+        if (p->chunk > kSpreadItemMax) {  // the spread's own work list, count in status[3]
+            k_scan_emit_chunks<<<emit_blocks, kItemScanThreads, 0, p->stream>>>(
+                p->cell_count, ntiles, g.T * g.T, kSpreadItemMax, p->items, item_state + item_words, p->d_status,
+                p->d_status + 3);
+            NFFT_TRY_CUDA(cudaGetLastError());
+        }
     }
     stage_end(p, ST_SORT);
     if (p->gather_auto) p->gather_variant = auto_gather(p, M);
@@ -2015,9 +2205,13 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
         p->points_valid = true;
         return NFFT2D_OK;
     }
-    const int *hs = p->h_status;  // page-locked: the read-back is one small DMA
-    NFFT_TRY_CUDA(cudaMemcpyAsync(p->h_status, p->d_status, 4 * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+    // the read-back is one small DMA, or the kernel's own write
+    if (!one) NFFT_TRY_CUDA(cudaMemcpyAsync(p->h_status, p->d_status, 4 * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     NFFT_TRY_CUDA(cudaStreamSynchronize(p->stream));
+    if (one && hs[0] < 0) {  // given up on at a barrier
+        NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status + kBarrierWord, 0, 2 * sizeof(int), p->stream));
+        return NFFT2D_ERR_DEVICE_TIMEOUT;
+    }
     if (hs[1] & kErrNonfinite) return NFFT2D_ERR_NONFINITE;
     if (hs[1] & kErrTimeout) return NFFT2D_ERR_DEVICE_TIMEOUT;
     if (hs[0] < 0 || hs[0] > p->chunks_cap) return NFFT2D_ERR_INTERNAL;

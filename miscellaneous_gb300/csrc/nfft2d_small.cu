@@ -32,7 +32,7 @@
 namespace nfft2d {
 namespace {
 
-constexpr int kSmallCtas = 128;    // all resident: one an SM
+constexpr int kSmallCtas = kGridCtas;
 constexpr int kSmallThreads = 128;
 constexpr int kSmallWarpsCta = kSmallThreads / 32;
 constexpr int kSmallWarps = kSmallCtas * kSmallWarpsCta;
@@ -44,40 +44,6 @@ struct SmallArgs {
     const float *d1, *d2;
     const float2 *tw1, *tw2;  // exp(-2 pi i m / n)
 };
-
-// What any CTA wrote before it arrived, every thread of the kernel sees after
-// the wait; `target`: the CTAs' arrivals so far.  False, latched, if the wait
-// runs out (the CTA leaves; so do the others, by their own waits).
-__device__ __forceinline__ void grid_arrive(int *status) {
-    __syncthreads();
-    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(status + kBarrierWord) : "memory");
-}
-__device__ __forceinline__ bool grid_wait(int *status, int target) {
-    __shared__ int ok;
-    if (threadIdx.x == 0) {
-        int seen = 0;
-        uint32_t spins = 0;
-        do
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(status + kBarrierWord) : "memory");
-        while (seen < target && ++spins < kSpinLimit);
-        ok = seen >= target;
-        if (!ok) latch_error(status, kErrTimeout);
-    }
-    __syncthreads();
-    return ok != 0;
-}
-__device__ __forceinline__ bool grid_barrier(int *status, int target) {
-    grid_arrive(status);
-    return grid_wait(status, target);
-}
-// The last CTA to come here leaves the barrier's words zero for the next launch.
-__device__ __forceinline__ void grid_done(int *status) {
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(status + kBarrierWord + 1, 1) == kSmallCtas - 1) {
-        status[kBarrierWord] = 0;
-        status[kBarrierWord + 1] = 0;
-    }
-}
 
 // Loads of what this kernel itself writes (never the read-only path).
 __device__ __forceinline__ float2 ld_rw(const float2 *p) {
