@@ -108,7 +108,11 @@ __global__ void k_batch_pad(const BatchDesc *__restrict__ d, int n, const BatchI
     }
 }
 
-__global__ void k_batch_crop(const BatchDesc *__restrict__ d, int n, const BatchIO *__restrict__ io) {
+// filt: a weight per output of every transform (the far-field step's spectral
+// filter), or null.  A weight here costs a load; its own pass over the outputs
+// read and wrote them again (10 us for 250 fields of 88^2).
+__global__ void k_batch_crop(const BatchDesc *__restrict__ d, int n, const BatchIO *__restrict__ io,
+                             const float *__restrict__ filt) {
     const int t = find_transform<2>(d, n, blockIdx.x);
     const BatchDesc &D = d[t];
     const int i = blockIdx.x - D.crop_base;
@@ -123,7 +127,13 @@ __global__ void k_batch_crop(const BatchDesc *__restrict__ d, int n, const Batch
         const int c = k2 < 0 ? k2 + n2 : k2;
         const float s = s1 * D.deap2[j];
         const float2 g = src[c];
-        F[static_cast<size_t>(i) * N2 + j] = make_float2(g.x * s, g.y * s);
+        float2 v = make_float2(g.x * s, g.y * s);
+        const size_t at = static_cast<size_t>(i) * N2 + j;
+        if (filt) {  // farFieldFiltering (Synthesis.cu:402)
+            const float w = __ldg(filt + at);
+            v = make_float2(w * v.x, w * v.y);
+        }
+        F[at] = v;
     }
 }
 
@@ -304,6 +314,8 @@ struct nfft2d_batch_s {
     };
     std::vector<Group> groups;
     BatchDesc *d_desc = nullptr;
+    BatchDesc *h_desc = nullptr;  // pinned; written while the batch's stream is idle
+    SmallBinSpace bin;
     BatchIO *d_io = nullptr;
     BatchIO *h_io = nullptr;  // pinned
     int *d_work = nullptr;    // spread work counter
@@ -339,6 +351,10 @@ void batch_free(nfft2d_batch_s *b) {
     for (auto *p : b->plans) release_plan(p);
     cudaFree(b->grids);
     cudaFree(b->d_desc);
+    cudaFreeHost(b->h_desc);
+    cudaFreeHost(b->bin.h_jobs);
+    cudaFree(b->bin.d_jobs);
+    cudaFreeHost(b->bin.h_out);
     cudaFree(b->d_io);
     cudaFreeHost(b->h_io);
     cudaFree(b->d_work);
@@ -443,7 +459,7 @@ int launch_spread_k(nfft2d_batch_s *b, const nfft2d_batch_s::KGroup &kg, int sms
 // type -1: the reference's spreading NFFT2_2D (type 1, sign -1).  The
 // elementwise stages and each size group's FFT cover all transforms at once;
 // the gather and the spread run once per window width.
-int enqueue(nfft2d_batch_s *b, int type) {
+int enqueue(nfft2d_batch_s *b, int type, const float *filter = nullptr) {
     const int n = b->count;
     int sms = 0, dev = 0;
     B_TRY(cudaGetDevice(&dev));
@@ -466,13 +482,16 @@ int enqueue(nfft2d_batch_s *b, int type) {
         B_TRY(cudaGetLastError());
         st = run_ffts(b, type == 1 ? CUFFT_INVERSE : CUFFT_FORWARD);
         if (st != NFFT2D_OK) return st;
-        k_batch_crop<<<b->total_crop, kThreads, 0, b->stream>>>(b->d_desc, n, b->d_io);
+        k_batch_crop<<<b->total_crop, kThreads, 0, b->stream>>>(b->d_desc, n, b->d_io, filter);
         B_TRY(cudaGetLastError());
     }
     return NFFT2D_OK;
 }
 
-int run(nfft2d_batch_s *b, int type, const void *const *in, void *const *out) {
+// once: launched as it is, not captured -- the points change before the next
+// run; `filter` weights the coefficients of a type -1 run.
+int run(nfft2d_batch_s *b, int type, const void *const *in, void *const *out, bool once = false,
+        const float *filter = nullptr) {
     if (!b || !in || !out) return NFFT2D_ERR_INVALID_ARG;
     if (!b->points_valid) return NFFT2D_ERR_NO_POINTS;
     // the point-side array of a transform with no points may be null
@@ -495,7 +514,7 @@ int run(nfft2d_batch_s *b, int type, const void *const *in, void *const *out) {
     B_TRY(cudaEventRecord(b->ev_io, b->stream));
     b->io_pending = true;
     const int gi = type == 2 ? 0 : (type == 1 ? 1 : 2);
-    if (b->use_graph) {
+    if (b->use_graph && !once) {
         if (!b->graph[gi]) {
             cudaGraph_t graph = nullptr;
             B_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
@@ -512,7 +531,7 @@ int run(nfft2d_batch_s *b, int type, const void *const *in, void *const *out) {
         }
         B_TRY(cudaGraphLaunch(b->graph[gi], b->stream));
     } else {
-        const int st = enqueue(b, type);
+        const int st = enqueue(b, type, filter);
         if (st != NFFT2D_OK) return st;
     }
     B_TRY(cudaEventRecord(b->ev_out, b->stream));
@@ -534,14 +553,6 @@ __global__ void k_scale_points(const float *const *__restrict__ X, const float *
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         xs[t * M + i] = x[i] * sx;  // vectorMulConstant<float>
         ys[t * M + i] = y[i] * sy;
-    }
-}
-__global__ void k_filter(float2 *const *__restrict__ F, const float *__restrict__ filt, long long n) {
-    float2 *f = F[blockIdx.y];
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const float w = filt[i];
-        f[i] = make_float2(w * f[i].x, w * f[i].y);  // farFieldFiltering
     }
 }
 }  // namespace
@@ -633,6 +644,10 @@ int nfft2d_batch_create_k(nfft2d_batch *out, int count, const int *N1, const int
         ++b->kgroups.back().n;
     }
     if (cudaMalloc(&b->d_desc, sizeof(BatchDesc) * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
+    if (cudaMallocHost(&b->h_desc, sizeof(BatchDesc) * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
+    if (cudaMallocHost(&b->bin.h_jobs, sizeof(SmallBinJob) * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
+    if (cudaMalloc(&b->bin.d_jobs, sizeof(SmallBinJob) * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
+    if (cudaMallocHost(&b->bin.h_out, sizeof(int) * 2 * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
     if (cudaMalloc(&b->d_io, sizeof(BatchIO) * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
     if (cudaMallocHost(&b->h_io, sizeof(BatchIO) * count) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
     if (cudaMalloc(&b->d_work, sizeof(int)) != cudaSuccess) return fail(NFFT2D_ERR_OOM);
@@ -656,9 +671,10 @@ int nfft2d_batch_destroy(nfft2d_batch b) {
     return NFFT2D_OK;
 }
 
-int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *const *x1, const void *const *x2,
-                            int coord_dtype, int units) {
-    if (!b || !M || !x1 || !x2) return NFFT2D_ERR_INVALID_ARG;
+// far: the far-field step's points -- device memory, scaled by c1 and c2 first;
+// NFFT2D_ERR_UNSUPPORTED when they don't bin in one launch.
+static int batch_set_points(nfft2d_batch b, const long long *M, const void *const *x1, const void *const *x2,
+                            int coord_dtype, int units, bool far, float c1, float c2) {
     b->points_valid = false;
     drop_graphs(b);
     B_TRY(cudaStreamSynchronize(b->stream));
@@ -676,8 +692,8 @@ int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *cons
             py[i] = x2[t];
         }
         int st = bin_small_batch(b->plans.data(), Mi.data(), px.data(), py.data(), coord_dtype, units, b->count,
-                                 b->stream);
-        if (st == NFFT2D_ERR_UNSUPPORTED) {
+                                 b->stream, b->bin, c1, c2, far);
+        if (st == NFFT2D_ERR_UNSUPPORTED && !far) {
             for (int i = 0; i < b->count; ++i) {
                 st = nfft2d_set_points_async(b->plans[i], Mi[i], px[i], py[i], coord_dtype, units);
                 if (st != NFFT2D_OK) return st;
@@ -692,7 +708,7 @@ int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *cons
             return st;
         }
     }
-    std::vector<BatchDesc> h(b->count);
+    BatchDesc *h = b->h_desc;  // the stream is idle: the last copy has left it
     int chunks = 0, rows = 0, crop = 0;
     long long points = 0, all_points = 0;
     for (int i = 0; i < b->count; ++i) {
@@ -722,8 +738,8 @@ int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *cons
         rows += p->g.n1;
         crop += p->N1;
     }
-    B_TRY(cudaMemcpy(b->d_desc, h.data(), sizeof(BatchDesc) * b->count, cudaMemcpyHostToDevice));
     if (all_points > 0x7fffffffLL) return NFFT2D_ERR_INVALID_ARG;  // global point indices are int
+    B_TRY(cudaMemcpyAsync(b->d_desc, h, sizeof(BatchDesc) * b->count, cudaMemcpyHostToDevice, b->stream));
     for (auto &kg : b->kgroups) {
         kg.chunk0 = h[kg.first].chunk_base;
         kg.point0 = h[kg.first].point_base;
@@ -739,6 +755,12 @@ int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *cons
     b->total_crop = crop;
     b->points_valid = true;
     return NFFT2D_OK;
+}
+
+int nfft2d_batch_set_points(nfft2d_batch b, const long long *M, const void *const *x1, const void *const *x2,
+                            int coord_dtype, int units) {
+    if (!b || !M || !x1 || !x2) return NFFT2D_ERR_INVALID_ARG;
+    return batch_set_points(b, M, x1, x2, coord_dtype, units, false, 1.f, 1.f);
 }
 
 int nfft2d_batch_forward(nfft2d_batch b, const void *const *F, void *const *f) { return run(b, 2, F, f); }
@@ -762,56 +784,41 @@ int nfft2d_batch_far_field(nfft2d_batch b, long long M, const float *const *X, c
     // the caller's coordinates were written on its stream
     B_TRY(cudaEventRecord(b->ev_in, b->user_stream));
     B_TRY(cudaStreamWaitEvent(b->stream, b->ev_in, 0));
-    float *xs = nullptr, *ys = nullptr;
-    const float **dxy = nullptr;
-    const size_t pts = static_cast<size_t>(n) * static_cast<size_t>(M);
-    B_TRY(cudaMallocAsync(&xs, sizeof(float) * pts + 16, b->stream));
-    B_TRY(cudaMallocAsync(&ys, sizeof(float) * pts + 16, b->stream));
-    B_TRY(cudaMallocAsync(&dxy, sizeof(float *) * 2 * n, b->stream));
-    std::vector<const float *> hxy(2 * static_cast<size_t>(n));
-    for (int i = 0; i < n; ++i) {
-        hxy[i] = X[i];
-        hxy[n + i] = Y[i];
-    }
-    int st = NFFT2D_OK;
-    if (cudaMemcpyAsync(dxy, hxy.data(), sizeof(float *) * 2 * n, cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
-        st = NFFT2D_ERR_CUDA;
-    if (st == NFFT2D_OK && M > 0) {
-        const dim3 grid(static_cast<unsigned>(std::min<long long>((M + 255) / 256, 64)), static_cast<unsigned>(n));
-        k_scale_points<<<grid, 256, 0, b->stream>>>(dxy, dxy + n, M, scale_x, scale_y, xs, ys);
-        if (cudaGetLastError() != cudaSuccess) st = NFFT2D_ERR_CUDA;
-    }
-    if (st == NFFT2D_OK) {
-        std::vector<long long> Ms(static_cast<size_t>(n), M);
-        std::vector<const void *> px(static_cast<size_t>(n)), py(static_cast<size_t>(n));
+    // the binning scales the coordinates as it reads them, the crop filters the
+    // fields as it writes them: no pass of their own
+    const std::vector<long long> Ms(static_cast<size_t>(n), M);
+    std::vector<const void *> px(X, X + n), py(Y, Y + n);
+    int st = batch_set_points(b, Ms.data(), px.data(), py.data(), NFFT2D_COORD_F32, NFFT2D_UNITS_GRID, true, scale_x,
+                              scale_y);
+    if (st == NFFT2D_ERR_UNSUPPORTED) {  // larger sets: scaled copies, binned per transform
+        float *xs = nullptr, *ys = nullptr;
+        const float **dxy = nullptr;
+        const size_t pts = static_cast<size_t>(n) * static_cast<size_t>(M);
+        B_TRY(cudaMallocAsync(&xs, sizeof(float) * pts + 16, b->stream));
+        B_TRY(cudaMallocAsync(&ys, sizeof(float) * pts + 16, b->stream));
+        B_TRY(cudaMallocAsync(&dxy, sizeof(float *) * 2 * n, b->stream));
+        std::vector<const void *> hxy(px);
+        hxy.insert(hxy.end(), py.begin(), py.end());
+        st = NFFT2D_OK;
+        if (cudaMemcpyAsync(dxy, hxy.data(), sizeof(float *) * 2 * n, cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
+            st = NFFT2D_ERR_CUDA;
+        if (st == NFFT2D_OK && M > 0) {
+            const dim3 grid(static_cast<unsigned>(std::min<long long>((M + 255) / 256, 64)), static_cast<unsigned>(n));
+            k_scale_points<<<grid, 256, 0, b->stream>>>(dxy, dxy + n, M, scale_x, scale_y, xs, ys);
+            if (cudaGetLastError() != cudaSuccess) st = NFFT2D_ERR_CUDA;
+        }
         for (int i = 0; i < n; ++i) {
             px[i] = xs + static_cast<size_t>(i) * M;
             py[i] = ys + static_cast<size_t>(i) * M;
         }
-        st = nfft2d_batch_set_points(b, Ms.data(), px.data(), py.data(), NFFT2D_COORD_F32, NFFT2D_UNITS_GRID);
+        if (st == NFFT2D_OK)
+            st = nfft2d_batch_set_points(b, Ms.data(), px.data(), py.data(), NFFT2D_COORD_F32, NFFT2D_UNITS_GRID);
+        cudaFreeAsync(xs, b->stream);
+        cudaFreeAsync(ys, b->stream);
+        cudaFreeAsync(dxy, b->stream);
     }
-    cudaFreeAsync(xs, b->stream);
-    cudaFreeAsync(ys, b->stream);
-    cudaFreeAsync(dxy, b->stream);
     if (st != NFFT2D_OK) return st;
-    if ((st = run(b, -1, excitations, far_field)) != NFFT2D_OK) return st;  // NFFT2_2D_GPU for every particle
-    if (filter && cells > 0) {
-        float2 **dF = nullptr;
-        B_TRY(cudaMallocAsync(&dF, sizeof(float2 *) * n, b->user_stream));
-        std::vector<float2 *> hF(static_cast<size_t>(n));
-        for (int i = 0; i < n; ++i) hF[i] = static_cast<float2 *>(far_field[i]);
-        const cudaError_t e = cudaMemcpyAsync(dF, hF.data(), sizeof(float2 *) * n, cudaMemcpyHostToDevice,
-                                              b->user_stream);
-        if (e == cudaSuccess) {
-            const dim3 grid(static_cast<unsigned>(std::min<long long>((cells + 255) / 256, 64)),
-                            static_cast<unsigned>(n));
-            k_filter<<<grid, 256, 0, b->user_stream>>>(dF, filter, cells);
-        }
-        cudaFreeAsync(dF, b->user_stream);
-        B_TRY(e);
-        B_TRY(cudaGetLastError());
-    }
-    return NFFT2D_OK;
+    return run(b, -1, excitations, far_field, true, filter);  // NFFT2_2D_GPU for every particle, filtered
 }
 
 int nfft2d_batch_set_graph(nfft2d_batch b, int on) {

@@ -248,6 +248,7 @@ void pooled_plan_release(cufftHandle h);
 struct SmallBinJob {
     const void *x1, *x2;  // DEVICE coordinates (FP32 or FP64 as the batch's call)
     int M;
+    float c1, c2;         // FP32 factors of the coordinates, before the reduction
     double s1, s2;        // sigma * unit scale per dimension
     float s1f, s2f;
     int exact;            // exact FP32 reduction (power-of-two scales, FP32 data)
@@ -259,17 +260,25 @@ struct SmallBinJob {
     int4 *chunks;
     int chunk;
     int *status;          // the plan's status words ([0] work items, [1] error bits)
-    int *out;             // work items and error bits, read back by the host
+    int *out;             // work items and error bits, page-locked, for the host
+};
+
+// A batch's own buffers for bin_small_batch, `count` entries each.
+struct SmallBinSpace {
+    SmallBinJob *h_jobs = nullptr, *d_jobs = nullptr;  // h_: page-locked
+    int *h_out = nullptr;                              // 2 a transform, page-locked, written by the kernel
 };
 
 // Bin the points of `count` FP32 plans (a batch's transforms) with one
 // launch: one CTA per transform with its cell counters in shared memory.
 // Same result as nfft2d_set_points on each plan (units: NFFT2D_UNITS_*);
-// synchronizes once.  NFFT2D_ERR_UNSUPPORTED when a plan's cells
-// do not fit in shared memory or a transform has more than 2^24 points
-// (the caller bins those per plan).
-int bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, const void *const *x1,
-                    const void *const *x2, int coord_dtype, int units, int count, cudaStream_t stream);
+// synchronizes once.  c1, c2: FP32 factors the coordinates are multiplied by
+// first; device_coords: x1, x2 are known to be readable by the device.
+// NFFT2D_ERR_UNSUPPORTED when a plan's cells do not fit in shared memory or a
+// transform has more than 2^24 points (the caller bins those per plan).
+int bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, const void *const *x1, const void *const *x2,
+                    int coord_dtype, int units, int count, cudaStream_t stream, const SmallBinSpace &space,
+                    float c1 = 1.f, float c2 = 1.f, bool device_coords = false);
 
 // After the plan's status words were copied to p->h_status and its stream
 // went idle: completes a set_points enqueued by nfft2d_set_points_async

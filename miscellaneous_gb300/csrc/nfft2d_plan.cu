@@ -990,8 +990,8 @@ __global__ void __launch_bounds__(kSmallBinThreads, 1) k_bin_small(const SmallBi
     for (int i = tid; i < J.M; i += kSmallBinThreads) {
         Rec32 r;
         int mu1, mu2;
-        const bool ok1 = reduce_coord(x1[i], 0.0, J.s1, J.s1f, J.exact != 0, g.n1, mu1, r.t1);
-        const bool ok2 = reduce_coord(x2[i], 0.0, J.s2, J.s2f, J.exact != 0, g.n2, mu2, r.t2);
+        const bool ok1 = reduce_coord(x1[i] * static_cast<CT>(J.c1), 0.0, J.s1, J.s1f, J.exact != 0, g.n1, mu1, r.t1);
+        const bool ok2 = reduce_coord(x2[i] * static_cast<CT>(J.c2), 0.0, J.s2, J.s2f, J.exact != 0, g.n2, mu2, r.t2);
         if (!ok1 || !ok2) {  // as k_bin_pass1: reported, and binned at cell 0 with t = 0
             bad = true;
             mu1 = mu2 = 0;
@@ -1955,12 +1955,12 @@ static int coord_device_ptr(const nfft2d_plan_s *p, const void *x, const void **
 
 extern "C++" {
 int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, const void *const *x1,
-                             const void *const *x2, int coord_dtype, int units, int count, cudaStream_t stream) {
+                             const void *const *x2, int coord_dtype, int units, int count, cudaStream_t stream,
+                             const SmallBinSpace &space, float c1, float c2, bool device_coords) {
     if (count < 1 || (coord_dtype != NFFT2D_COORD_F32 && coord_dtype != NFFT2D_COORD_F64))
         return NFFT2D_ERR_INVALID_ARG;
     if (units != NFFT2D_UNITS_GRID && units != NFFT2D_UNITS_UNIT && units != NFFT2D_UNITS_RADIANS)
         return NFFT2D_ERR_INVALID_ARG;
-    std::vector<SmallBinJob> jobs(static_cast<size_t>(count));
     size_t max_cells = 0;
     for (int i = 0; i < count; ++i) {
         nfft2d_plan_s *p = plans[i];
@@ -1970,12 +1970,10 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
     }
     const size_t smem = sizeof(unsigned) * (max_cells + 1 + 32);
     if (smem > 200 * 1024) return NFFT2D_ERR_UNSUPPORTED;  // the counters must fit in shared memory
-    int *d_out = nullptr;
-    SmallBinJob *d_jobs = nullptr;
     for (int i = 0; i < count; ++i) {
         nfft2d_plan_s *p = plans[i];
         const void *dx1 = x1[i], *dx2 = x2[i];
-        if (M[i] > 0) {
+        if (M[i] > 0 && !device_coords) {
             int st = coord_device_ptr(p, x1[i], &dx1);
             if (st == NFFT2D_OK) st = coord_device_ptr(p, x2[i], &dx2);
             if (st != NFFT2D_OK) return st;
@@ -1994,10 +1992,12 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
         p->xscale2 = s2;
         int e1 = 0, e2 = 0;
         const bool pow2 = std::frexp(s1, &e1) == 0.5 && std::frexp(s2, &e2) == 0.5;
-        SmallBinJob &J = jobs[static_cast<size_t>(i)];
+        SmallBinJob &J = space.h_jobs[i];
         J.x1 = dx1;
         J.x2 = dx2;
         J.M = static_cast<int>(M[i]);
+        J.c1 = c1;
+        J.c2 = c2;
         J.s1 = s1;
         J.s2 = s2;
         J.s1f = static_cast<float>(s1);
@@ -2011,31 +2011,20 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
         J.chunks = p->chunks;
         J.chunk = p->chunk;
         J.status = p->d_status;
-        J.out = nullptr;  // set below
+        J.out = space.h_out + 2 * i;
+        J.out[0] = -1;  // until the kernel has the counts
+        J.out[1] = 0;
     }
-    NFFT_TRY_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&d_out), sizeof(int) * 2 * count, stream));
-    for (int i = 0; i < count; ++i) jobs[static_cast<size_t>(i)].out = d_out + 2 * i;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&d_jobs), sizeof(SmallBinJob) * count, stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(SmallBinJob) * count, cudaMemcpyHostToDevice, stream);
+    NFFT_TRY_CUDA(cudaMemcpyAsync(space.d_jobs, space.h_jobs, sizeof(SmallBinJob) * count, cudaMemcpyHostToDevice, stream));
     auto kernel = coord_dtype == NFFT2D_COORD_F64 ? k_bin_small<double> : k_bin_small<float>;
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess) {
-        kernel<<<count, kSmallBinThreads, smem, stream>>>(d_jobs);
-        e = cudaGetLastError();
-    }
-    std::vector<int> out(static_cast<size_t>(2 * count));
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out.data(), d_out, sizeof(int) * 2 * count, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    cudaFreeAsync(d_jobs, stream);
-    cudaFreeAsync(d_out, stream);
-    if (e != cudaSuccess) return status_from_cuda(e);
+    NFFT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kernel<<<count, kSmallBinThreads, smem, stream>>>(space.d_jobs);
+    NFFT_TRY_CUDA(cudaGetLastError());
+    NFFT_TRY_CUDA(cudaStreamSynchronize(stream));
     int status = NFFT2D_OK;
     for (int i = 0; i < count; ++i) {
         nfft2d_plan_s *p = plans[i];
-        const int n_chunks = out[static_cast<size_t>(2 * i)], bits = out[static_cast<size_t>(2 * i + 1)];
+        const int n_chunks = space.h_out[2 * i], bits = space.h_out[2 * i + 1];
         if (bits & kErrNonfinite) {
             status = NFFT2D_ERR_NONFINITE;
             continue;

@@ -19,7 +19,10 @@ units, both signs, gradients, timing).
 """
 from __future__ import annotations
 
+import array
 import ctypes
+import itertools
+import operator
 import threading
 
 import torch
@@ -47,6 +50,23 @@ def _require_cuda(t: torch.Tensor, name: str, dtype: torch.dtype, numel: int | N
     if numel is not None and t.numel() != numel:
         raise ValueError(f"{name} must have {numel} elements, got {t.numel()}")
     return t
+
+
+_dtype_of, _on_cuda = operator.attrgetter("dtype"), operator.attrgetter("is_cuda")
+
+
+def _require_all(ts, name: str, dtype: torch.dtype, numels) -> None:
+    """_require_cuda of every tensor of a list (numels: one count, or one per
+    tensor).  Each property is first read of all tensors at once: five
+    calls a tensor took 0.3 us, 230 us for a swarm's 750 tensors."""
+    same = isinstance(numels, int)
+    if (set(map(type, ts)) <= {torch.Tensor} and set(map(_dtype_of, ts)) <= {dtype} and all(map(_on_cuda, ts))
+            and all(map(torch.Tensor.is_contiguous, ts))):
+        got = map(torch.Tensor.numel, ts)
+        if (set(got) <= {numels}) if same else (list(got) == numels):
+            return
+    for t, n in zip(ts, itertools.repeat(numels) if same else numels):
+        _require_cuda(t, name, dtype, n)
 
 
 class Plan:
@@ -300,7 +320,11 @@ class Batch:
 
     @staticmethod
     def _ptrs(ts):
-        return (ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
+        try:
+            ptrs = list(map(torch.Tensor.data_ptr, ts))
+        except TypeError:  # something else with a data_ptr()
+            ptrs = [t.data_ptr() for t in ts]
+        return (ctypes.c_void_p * len(ptrs)).from_buffer(array.array("Q", ptrs))
 
     def set_points(self, x1s, x2s, units: str = "unit") -> None:
         if len(x1s) != self.count or len(x2s) != self.count:
@@ -319,16 +343,16 @@ class Batch:
         self._keep = (list(x1s), list(x2s))
 
     def forward(self, Fs, outs=None):
-        for (n1, n2), F in zip(self.sizes, Fs):
-            _require_cuda(F, "F", torch.complex64, n1 * n2)
+        Fs = list(Fs)
+        _require_all(Fs, "F", torch.complex64, [n1 * n2 for n1, n2 in self.sizes])
         if outs is None:
             outs = [torch.empty(m, dtype=torch.complex64, device=Fs[0].device) for m in self.M]
         check(self._lib.nfft2d_batch_forward(self._h, self._ptrs(Fs), self._ptrs(outs)), "nfft2d_batch_forward")
         return outs
 
     def adjoint(self, fs, outs=None):
-        for m, f in zip(self.M, fs):
-            _require_cuda(f, "f", torch.complex64, m)
+        fs = list(fs)
+        _require_all(fs, "f", torch.complex64, self.M)
         if outs is None:
             outs = [torch.empty(n1 * n2, dtype=torch.complex64, device=fs[0].device) for n1, n2 in self.sizes]
         check(self._lib.nfft2d_batch_adjoint(self._h, self._ptrs(fs), self._ptrs(outs)), "nfft2d_batch_adjoint")
@@ -336,8 +360,8 @@ class Batch:
 
     def spread_ref(self, fs, outs=None):
         """Type 1 with the reference's sign (NFFT2_2D_GPU) for every transform."""
-        for m, f in zip(self.M, fs):
-            _require_cuda(f, "f", torch.complex64, m)
+        fs = list(fs)
+        _require_all(fs, "f", torch.complex64, self.M)
         if outs is None:
             outs = [torch.empty(n1 * n2, dtype=torch.complex64, device=fs[0].device) for n1, n2 in self.sizes]
         check(self._lib.nfft2d_batch_spread_ref(self._h, self._ptrs(fs), self._ptrs(outs)), "nfft2d_batch_spread_ref")
@@ -352,11 +376,11 @@ class Batch:
         and the spectral filter (float32, N1*N2).  Returns the far fields."""
         if len(X) != self.count or len(Y) != self.count or len(excitations) != self.count:
             raise ValueError("one X, Y and excitation per transform")
+        X, Y, excitations = list(X), list(Y), list(excitations)
         M = X[0].numel()
-        for a, b, e in zip(X, Y, excitations):
-            _require_cuda(a, "X", torch.float32, M)
-            _require_cuda(b, "Y", torch.float32, M)
-            _require_cuda(e, "excitations", torch.complex64, M)
+        _require_all(X, "X", torch.float32, M)
+        _require_all(Y, "Y", torch.float32, M)
+        _require_all(excitations, "excitations", torch.complex64, M)
         if filter is not None:
             n1, n2 = self.sizes[0]
             _require_cuda(filter, "filter", torch.float32, n1 * n2)
@@ -366,7 +390,7 @@ class Batch:
                                                float(scale_y), self._ptrs(excitations),
                                                _ptr(filter), self._ptrs(outs)), "nfft2d_batch_far_field")
         self.M = [M] * self.count
-        self._keep = (list(X), list(Y))
+        self._keep = (X, Y)
         return outs
 
     def synchronize(self) -> None:
