@@ -316,6 +316,7 @@ cudaError_t fused_type1_cols(const nfft2d_plan_s *p, int sign, void *F);
 
 // Whole transforms in one launch (nfft2d_small.cu): whether the plan's sizes
 // and the device take them, and the launches (points set).
+constexpr int kSmallCells = 256 * 256;
 bool small_available(const nfft2d_plan_s *p);
 cudaError_t launch_small_type2(const nfft2d_plan_s *p, int sign, const void *F, void *f);
 cudaError_t launch_small_type1(const nfft2d_plan_s *p, int sign, const void *f, void *F);

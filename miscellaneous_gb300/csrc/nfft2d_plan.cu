@@ -383,7 +383,7 @@ bool use_small(const nfft2d_plan_s *p, bool adjoint) {
         p->timer.on || p->g.T != 16 || p->g.SW != spread_strip_width(p->K) || p->chunk > kSpreadItemMax)
         return false;
     const long long cells = 1LL * p->g.n1 * p->g.n2;
-    return cells <= 256 * 256 && p->M <= (adjoint ? 1 << 15 : cells <= 128 * 128 ? 1 << 14 : 1 << 13);
+    return p->M <= (adjoint ? 1 << 15 : cells <= 128 * 128 ? 1 << 14 : 1 << 13);
 }
 
 // The automatic FP32 gather: the direct 16-byte-load gather from 128 points

@@ -141,7 +141,7 @@ struct SmallPatch {
 };
 
 // Shared memory: the twiddles, then a warp's two FFT buffers or its patch.
-constexpr int kTwBytes = 2 * kSmallSide * 8;
+constexpr int kTwBytes = (kSmallSide + kSmallCells / kSmallSide) * 8;  // the longest pair of sides
 template <int K>
 constexpr int small_warp_bytes() {
     return std::max(2 * kSmallSide * 8, SmallPatch<K>::BYTES);
@@ -447,15 +447,11 @@ SmallArgs small_args(const nfft2d_plan_s *p, int sign) {
     return a;
 }
 
-// A cooperative launch.  query: whether all CTAs fit the device at once.
 template <typename Kernel, typename... Args>
-cudaError_t launch_grid(Kernel kernel, int smem, const nfft2d_plan_s *p, bool query, Args... args) {
-    if (query) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        int n = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kSmallThreads, smem);
-        if (e == cudaSuccess && n * p->num_sms < kSmallCtas) e = cudaErrorNotSupported;
-        return e;
+cudaError_t launch_grid(Kernel kernel, int smem, const nfft2d_plan_s *p, Args... args) {
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
     }
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeCooperative;
@@ -471,16 +467,16 @@ cudaError_t launch_grid(Kernel kernel, int smem, const nfft2d_plan_s *p, bool qu
 }
 
 template <int K>
-cudaError_t type2_K(const nfft2d_plan_s *p, int sign, const void *F, void *f, bool query) {
-    return launch_grid(k_small_type2<K>, small_smem<K>(), p, query, static_cast<const float2 *>(F),
+cudaError_t type2_K(const nfft2d_plan_s *p, int sign, const void *F, void *f) {
+    return launch_grid(k_small_type2<K>, small_smem<K>(), p, static_cast<const float2 *>(F),
                        static_cast<float2 *>(p->grid), static_cast<const Rec32 *>(p->recs),
                        static_cast<const int4 *>(p->chunks), static_cast<float2 *>(f), small_args(p, sign),
                        make_kargs(p));
 }
 
 template <int K>
-cudaError_t type1_K(const nfft2d_plan_s *p, int sign, const void *f, void *F, bool query) {
-    return launch_grid(k_small_type1<K>, small_smem<K>(), p, query, p->tmap, static_cast<const float2 *>(f),
+cudaError_t type1_K(const nfft2d_plan_s *p, int sign, const void *f, void *F) {
+    return launch_grid(k_small_type1<K>, small_smem<K>(), p, p->tmap, static_cast<const float2 *>(f),
                        static_cast<float2 *>(p->grid), static_cast<const Rec32 *>(p->recs),
                        static_cast<const int4 *>(p->chunks), static_cast<float2 *>(F), small_args(p, sign),
                        make_kargs(p));
@@ -503,22 +499,18 @@ cudaError_t by_width(int K, Fn fn) {
 }  // namespace
 
 bool small_available(const nfft2d_plan_s *p) {
-    if (p->precision != NFFT2D_F32 || p->grid_external || !p->fused_ok || !p->tmap_ok) return false;
-    if (p->g.n1 > kSmallSide || p->g.n2 > kSmallSide || p->g.T != kRegTile) return false;
-    const bool ok = by_width(p->K, [&](auto k) {
-                        const cudaError_t e = type2_K<decltype(k)::value>(p, -1, nullptr, nullptr, true);
-                        return e != cudaSuccess ? e : type1_K<decltype(k)::value>(p, -1, nullptr, nullptr, true);
-                    }) == cudaSuccess;
-    if (!ok) cudaGetLastError();
-    return ok;
+    // power-of-two sides (fused_ok); a CTA an SM, all of them resident
+    const Geom &g = p->g;
+    return p->precision == NFFT2D_F32 && !p->grid_external && p->fused_ok && p->tmap_ok && g.T == kRegTile &&
+           g.n1 <= kSmallSide && g.n2 <= kSmallSide && 1LL * g.n1 * g.n2 <= kSmallCells && p->num_sms >= kSmallCtas;
 }
 
 cudaError_t launch_small_type2(const nfft2d_plan_s *p, int sign, const void *F, void *f) {
-    return by_width(p->K, [&](auto k) { return type2_K<decltype(k)::value>(p, sign, F, f, false); });
+    return by_width(p->K, [&](auto k) { return type2_K<decltype(k)::value>(p, sign, F, f); });
 }
 
 cudaError_t launch_small_type1(const nfft2d_plan_s *p, int sign, const void *f, void *F) {
-    return by_width(p->K, [&](auto k) { return type1_K<decltype(k)::value>(p, sign, f, F, false); });
+    return by_width(p->K, [&](auto k) { return type1_K<decltype(k)::value>(p, sign, f, F); });
 }
 
 }  // namespace nfft2d
