@@ -494,26 +494,31 @@ bool fused_fft_eligible(int precision, int n1, int n2) {
 }
 
 int setup_fused_fft(nfft2d_plan_s *p) {
-    if (p->tw1 || p->tw2) cudaStreamSynchronize(p->stream);  // no transform on the old tables in flight
+    if (p->tw1) cudaStreamSynchronize(p->stream);  // no transform on the old tables in flight
     plan_free(p->tw1);
-    plan_free(p->tw2);
     p->tw1 = p->tw2 = nullptr;
-    p->fused_ok = false;
-    if (!fused_fft_eligible(p->precision, p->g.n1, p->g.n2)) return NFFT2D_OK;
-    for (int d = 0; d < 2; ++d) {
-        const int n = d == 0 ? p->g.n1 : p->g.n2;
-        std::vector<float2> h(n);
-        for (int m = 0; m < n; ++m) {
+    p->fused_ok = p->mixed_ok = false;
+    const int n1 = p->g.n1, n2 = p->g.n2;
+    const bool fused = fused_fft_eligible(p->precision, n1, n2);
+    const bool mixed = p->strips && mixed_fft_eligible(p->precision, n1, n2);
+    if (!fused && !mixed) return NFFT2D_OK;
+    // both tables in one buffer; from the first quarter, as far as n has quarters
+    std::vector<float2> h(static_cast<size_t>(n1) + (n1 != n2 ? n2 : 0));
+    for (int at = 0, n = n1; at < static_cast<int>(h.size()); at += n, n = n2) {
+        const int quarter = n % 4 == 0 ? n / 4 : n;
+        for (int m = 0; m < quarter; ++m) {
             const double ang = -2.0 * 3.141592653589793238462643383279502884 * m / n;
-            h[m] = make_float2(static_cast<float>(std::cos(ang)), static_cast<float>(std::sin(ang)));
+            h[at + m] = make_float2(static_cast<float>(std::cos(ang)), static_cast<float>(std::sin(ang)));
         }
-        float2 **dst = d == 0 ? &p->tw1 : &p->tw2;
-        if (plan_malloc(reinterpret_cast<void **>(dst), sizeof(float2) * n) != cudaSuccess) return NFFT2D_ERR_OOM;
-        if (cudaMemcpyAsync(*dst, h.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, p->stream) != cudaSuccess ||
-            cudaStreamSynchronize(p->stream) != cudaSuccess)
-            return NFFT2D_ERR_CUDA;
+        for (int m = quarter; m < n; ++m) h[at + m] = make_float2(h[at + m - quarter].y, -h[at + m - quarter].x);
     }
-    p->fused_ok = true;
+    if (plan_malloc(reinterpret_cast<void **>(&p->tw1), sizeof(float2) * h.size()) != cudaSuccess) return NFFT2D_ERR_OOM;
+    p->tw2 = p->tw1 + (n1 != n2 ? n1 : 0);
+    if (cudaMemcpyAsync(p->tw1, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice, p->stream) != cudaSuccess ||
+        cudaStreamSynchronize(p->stream) != cudaSuccess)
+        return NFFT2D_ERR_CUDA;
+    p->fused_ok = fused;
+    p->mixed_ok = mixed;
     return NFFT2D_OK;
 }
 

@@ -175,8 +175,9 @@ struct nfft2d_plan_s {
     bool pruned_ok = false;
     int fft_mode = -1;                       // -1 auto, 0 2D plan, 1 pruned passes, 2 fused passes
     bool fused_ok = false;                   // twiddle tables of the fused passes are set up
+    bool mixed_ok = false;                   // as fused_ok, for sides of small prime factors
     bool small_ok = false;                   // the one-launch transforms fit the plan and the device
-    float2 *tw1 = nullptr, *tw2 = nullptr;   // exp(-2 pi i m / n1), exp(-2 pi i m / n2)
+    float2 *tw1 = nullptr, *tw2 = nullptr;   // exp(-2 pi i m / n1), exp(-2 pi i m / n2), one buffer
     CUtensorMap tmap;  // 64-byte aligned by its own declaration
     CUtensorMap tmap_spread;  // box of one strip patch of the FP32 tiled spread
     bool tmap_ok = false;
@@ -313,6 +314,13 @@ cudaError_t fused_type2_cols(const nfft2d_plan_s *p, int sign, const void *F);
 cudaError_t fused_type2_rows(const nfft2d_plan_s *p, int sign);
 cudaError_t fused_type1_rows(const nfft2d_plan_s *p, int sign);
 cudaError_t fused_type1_cols(const nfft2d_plan_s *p, int sign, void *F);
+
+// The same passes for sides of small prime factors (nfft2d_fft_mixed.cu).
+bool mixed_fft_eligible(int precision, int n1, int n2);
+cudaError_t mixed_type2_cols(const nfft2d_plan_s *p, int sign, const void *F);
+cudaError_t mixed_type2_rows(const nfft2d_plan_s *p, int sign);
+cudaError_t mixed_type1_rows(const nfft2d_plan_s *p, int sign);
+cudaError_t mixed_type1_cols(const nfft2d_plan_s *p, int sign, void *F);
 
 // Whole transforms in one launch (nfft2d_small.cu): whether the plan's sizes
 // and the device take them, and the launches (points set).

@@ -366,6 +366,29 @@ bool use_fused(const nfft2d_plan_s *p) {
     return p->fft_mode < 0 && 1LL * p->g.n1 * p->g.n2 < 2048LL * 2048LL;
 }
 
+// The same passes with sides of small prime factors (nfft2d_fft_mixed.cu), in
+// automatic mode, where the fused ones do not run: below 2048 x 2048 cells,
+// and above where both sides have a prime factor of 5 or more (powers of 2 and
+// 3 are what cuFFT is best at).  Not for a regridder's plan (no strips), which
+// pads by itself.  Measured on GB300, w 6, 50 k points, coefficients, us, cuFFT
+// with its separate kernels -> here (forward | adjoint):
+//     50 x 50    25.5 -> 18.9 | 41.3 -> 39.0      250 x 378   36.9 -> 27.1 | 45.2 -> 37.0
+//    500 x 500   39.0 -> 34.9 | 53.4 -> 49.9      630 x 630   66.6 -> 53.3 | 81.7 -> 71.8
+//   1100 x 900    136 -> 96   |  153 -> 116      1000 x 1000   120 -> 98   |  131 -> 124
+//   1100 x 1300   222 -> 137  |  234 -> 165      1920 x 1920   366 -> 306  |  394 -> 384
+//   1536 x 1536   241 -> 231  |  234 -> 254      1050 x 1024   111 -> 107  |  127 -> 134
+//   1024 x 1024    94 -> 100  |  111 -> 126      2048 x 2048   274 -> 362  |  320 -> 462
+// (the last four stay with cuFFT).  Errors fall, 2.5e-7 .. 3.7e-7 -> 2.0e-7.
+bool use_mixed(const nfft2d_plan_s *p) {
+    if (!p->mixed_ok || p->fft_mode >= 0 || use_fused(p)) return false;
+    auto rest = [](int n) {
+        for (const int f : {2, 3})
+            while (n % f == 0) n /= f;
+        return n;
+    };
+    return 1LL * p->g.n1 * p->g.n2 < 2048LL * 2048LL || (rest(p->g.n1) > 1 && rest(p->g.n2) > 1);
+}
+
 // Whole transforms in one launch (nfft2d_small.cu) for small sets on small
 // grids, where launches and latency are most of the time: with the plan's own
 // choice of stages, and no stage to time.  Measured on GB300, one launch
@@ -398,7 +421,7 @@ int auto_gather(const nfft2d_plan_s *p, long long M) {
 }
 
 int fft_mode_in_use(const nfft2d_plan_s *p) {
-    if (use_fused(p)) return 2;
+    if (use_fused(p) || use_mixed(p)) return 2;
     const bool pruned = p->fft_mode == 1 || (p->fft_mode < 0 && 1LL * p->g.n1 * p->g.n2 >= 2048LL * 2048LL);
     return pruned && p->pruned_ok ? 1 : 0;
 }
@@ -1275,7 +1298,6 @@ void destroy_plan(nfft2d_plan_s *p) {
     plan_free(p->d_status);
     plan_free_host(p->h_status, 4 * sizeof(int));
     plan_free(p->tw1);
-    plan_free(p->tw2);
     plan_free(p->cell_count);
     plan_free(p->scan_tmp);
     for (auto &e : p->timer.ev)
@@ -1330,8 +1352,8 @@ int check_plan(nfft2d_plan_s *p) { return p ? NFFT2D_OK : NFFT2D_ERR_INVALID_ARG
 // points (contiguous, pitch C) and N2/2 columns of n1 points (stride C), run
 // once per half of the band -- with the 2D plan as the fallback.  Nothing
 // for the fused passes.  Plans for a batch's external grid are the batch's.
-int ensure_ffts(nfft2d_plan_s *p) {
-    if (p->grid_external || use_fused(p)) return NFFT2D_OK;
+int ensure_ffts(nfft2d_plan_s *p, bool needed = false) {
+    if (p->grid_external || (!needed && (use_fused(p) || use_mixed(p)))) return NFFT2D_OK;
     const Geom &g = p->g;
     const cufftType t = p->precision == NFFT2D_F64 ? CUFFT_Z2Z : CUFFT_C2C;
     const bool pruned = p->fft_mode == 1 || (p->fft_mode < 0 && 1LL * g.n1 * g.n2 >= 2048LL * 2048LL);
@@ -1601,7 +1623,7 @@ int run_fft(nfft2d_plan_s *p, int sign, bool type2) {
     // vs 30 us; 2048^2: 40 vs 35 us; 4096^2: 153 vs 112 us)
     const bool pruned = p->fft_mode == 1 || (p->fft_mode < 0 && 1LL * g.n1 * g.n2 >= 2048LL * 2048LL);
     if (!(pruned && p->pruned_ok) && !p->fft_ok) {  // a mode set on a plan made without its plans
-        const int st = ensure_ffts(p);
+        const int st = ensure_ffts(p, true);
         if (st != NFFT2D_OK) return st;
     }
     if (!(pruned && p->pruned_ok)) return status_from_cufft(exec_at(p, p->fft, off, dir));
@@ -1619,12 +1641,12 @@ int run_fft(nfft2d_plan_s *p, int sign, bool type2) {
 
 
 int type2_prepare(nfft2d_plan_s *p, int sign, const void *F) {
-    if (use_fused(p)) {  // pad + band-column FFT, then row FFT + halo fill
+    if (use_fused(p) || use_mixed(p)) {  // pad + band-column FFT, then row FFT + halo fill
         stage_begin(p, ST_PAD);
-        NFFT_TRY_CUDA(fused_type2_cols(p, sign, F));
+        NFFT_TRY_CUDA(use_fused(p) ? fused_type2_cols(p, sign, F) : mixed_type2_cols(p, sign, F));
         stage_end(p, ST_PAD);
         stage_begin(p, ST_FFT2);
-        NFFT_TRY_CUDA(fused_type2_rows(p, sign));
+        NFFT_TRY_CUDA(use_fused(p) ? fused_type2_rows(p, sign) : mixed_type2_rows(p, sign));
         stage_end(p, ST_FFT2);
         return NFFT2D_OK;
     }
@@ -2273,12 +2295,12 @@ static int nfft2d_type1_impl(nfft2d_plan p, int sign, const void *f, void *F) {
     NFFT_TRY_CUDA(cudaMemsetAsync(p->grid, 0, cplx_size(p->precision) * static_cast<size_t>(g.Ra) * g.C, p->stream));
     NFFT_TRY_CUDA(launch_spread(p, f));
     stage_end(p, ST_SPREAD);
-    if (use_fused(p)) {  // fold + row FFT, then band-column FFT + crop
+    if (use_fused(p) || use_mixed(p)) {  // fold + row FFT, then band-column FFT + crop
         stage_begin(p, ST_FOLD);
-        NFFT_TRY_CUDA(fused_type1_rows(p, sign));
+        NFFT_TRY_CUDA(use_fused(p) ? fused_type1_rows(p, sign) : mixed_type1_rows(p, sign));
         stage_end(p, ST_FOLD);
         stage_begin(p, ST_FFT1);
-        NFFT_TRY_CUDA(fused_type1_cols(p, sign, F));
+        NFFT_TRY_CUDA(use_fused(p) ? fused_type1_cols(p, sign, F) : mixed_type1_cols(p, sign, F));
         stage_end(p, ST_FFT1);
         return NFFT2D_OK;
     }
