@@ -1,5 +1,5 @@
 // nfft2d_fft_mixed.cu -- the fused FFT passes (nfft2d_fft.cu) for sides that
-// are products of 2, 3, 5, 7, 11 and 13: FP32 plans whose oversampled grid is
+// are products of 2, 3, 5, 7, 11 and 13, with one larger prime: FP32 plans whose oversampled grid is
 // not a power of two a side, which otherwise run pad, a 2D library plan (two
 // kernels), halo fill -- fold, two, crop the other way.
 //
@@ -24,12 +24,13 @@ namespace nfft2d {
 namespace {
 
 constexpr int kMaxStages = 10;  // 4096 >= 3^7
-constexpr int kMixedMaxSide = 4096;
+constexpr int kMixedMaxSide = 4096, kMixedMaxPrime = 67;
 
 struct MixedFft {
     int n, stages;
     int radix[kMaxStages], done[kMaxStages];  // factor; product of the factors before it
     unsigned inv[kMaxStages];                 // ceil(2^32 / done): i / done for i < 2^16
+    unsigned inv_nb;                          // the same for n / radix[0]
 };
 
 struct MixedArgs {
@@ -224,6 +225,32 @@ __device__ __forceinline__ void any_stage(const MixedArgs &a, int i, const float
     }
 }
 
+// The first stage (L = 1) of a prime radix p above 13, between the buffers: a
+// thread computes output g and p - g of a butterfly from the sums and
+// differences of its inputs r and p - r.
+__device__ __forceinline__ void prime_stage(const MixedArgs &a, const float2 *__restrict__ tw, const float2 *u, float2 *v) {
+    const int p = a.f.radix[0], nb = a.f.n / p, P = a.logP;
+    const float s = a.s;
+    for (int i = threadIdx.x; i < (p / 2 + 1) * nb << P; i += blockDim.x) {
+        const int q = i & ((1 << P) - 1), e = i >> P;
+        const int g = static_cast<int>(__umulhi(static_cast<unsigned>(e), a.f.inv_nb)), b = e - g * nb;
+        float2 x = u[padded((b << P) + q)], y = make_float2(0.f, 0.f);
+        int m = 0;  // r g mod p
+#pragma unroll 4
+        for (int r = 1; r <= p / 2; ++r) {
+            m += g;
+            m -= m >= p ? p : 0;
+            const float2 w = __ldg(tw + m * nb);  // cos, -sin
+            const float2 c = u[padded(((b + r * nb) << P) + q)], d = u[padded(((b + (p - r) * nb) << P) + q)];
+            x = make_float2(fmaf(w.x, c.x + d.x, x.x), fmaf(w.x, c.y + d.y, x.y));
+            y = make_float2(fmaf(w.y, c.x - d.x, y.x), fmaf(w.y, c.y - d.y, y.y));
+        }
+        const float2 z = mul_si(y, -s);
+        v[padded(((b * p + g) << P) + q)] = cadd(x, z);
+        if (g) v[padded(((b * p + p - g) << P) + q)] = csub(x, z);
+    }
+}
+
 // The transform of P sequences from load(i, q) to store(i, q, value), between
 // two buffers of shared memory (element i of sequence q at i P + q): the first
 // stage reads and the last writes global memory (at least two stages).
@@ -232,7 +259,17 @@ __device__ __forceinline__ void mixed_fft(float2 *u, const MixedArgs &a, const f
                                           Store store) {
     const int P = a.logP;
     float2 *v = u + padded(a.f.n << P);
-    any_stage<true>(a, 0, tw, load, [=](int i, int q, float2 x) { u[padded((i << P) + q)] = x; });
+    if (a.f.radix[0] > 16) {
+#pragma unroll 4
+        for (int e = threadIdx.x; e < a.f.n << P; e += blockDim.x) u[padded(e)] = load(e >> P, e & ((1 << P) - 1));
+        __syncthreads();
+        prime_stage(a, tw, u, v);
+        float2 *t = u;
+        u = v;
+        v = t;
+    } else {
+        any_stage<true>(a, 0, tw, load, [=](int i, int q, float2 x) { u[padded((i << P) + q)] = x; });
+    }
     __syncthreads();
 #pragma unroll 1
     for (int st = 1; st + 1 < a.f.stages; ++st) {
@@ -355,22 +392,37 @@ __global__ void __launch_bounds__(kMixedThreads) k_mixed_cols_crop(const float2 
         });
 }
 
-// The factors of n, largest first; false if another prime is among them.
+// The factors of n, one prime from 17 to kMixedMaxPrime first, then largest
+// first; false if n has others.
 bool factor(int n, MixedFft *f) {
     *f = MixedFft{};
     f->n = n;
     int left = n, L = 1;
+    auto take = [&](int r) {
+        f->radix[f->stages] = r;
+        f->done[f->stages] = L;
+        f->inv[f->stages] = static_cast<unsigned>((0x100000000ull + L - 1) / L);
+        ++f->stages;
+        L *= r;
+        left /= r;
+    };
+    int rest = n;
+    for (const int r : {2, 3, 5, 7, 11, 13})
+        while (rest % r == 0) rest /= r;
+    if (rest > 1) {
+        for (int d = 17; d * d <= rest; d += 2)
+            if (rest % d == 0) return false;  // two of them
+        if (rest > kMixedMaxPrime) return false;
+        take(rest);
+    }
     for (const int r : {16, 13, 11, 9, 8, 7, 5, 4, 3, 2})
         while (left % r == 0) {
             if (f->stages == kMaxStages) return false;
-            f->radix[f->stages] = r;
-            f->done[f->stages] = L;
-            f->inv[f->stages] = static_cast<unsigned>((0x100000000ull + L - 1) / L);
-            ++f->stages;
-            L *= r;
-            left /= r;
+            take(r);
         }
-    return left == 1;
+    const int nb = n / f->radix[0];
+    f->inv_nb = static_cast<unsigned>((0x100000000ull + nb - 1) / nb);
+    return left == 1 && f->stages > 1;
 }
 
 MixedArgs mixed_args(const nfft2d_plan_s *p, int sign, int n) {
@@ -411,9 +463,17 @@ cudaError_t launch(Kernel kernel, const nfft2d_plan_s *p, int blocks, int elems,
 
 }  // namespace
 
+// A prime above 13 costs its own length per element: up to 2^20 cells it beats
+// cuFFT's chirp transforms.  Measured on GB300, w 6, 50 k points, coefficients
+// (primes), us, cuFFT -> here (forward | adjoint):
+//    106 x 134  (53, 67)  38.7 -> 26.7 | 54.6 -> 44.1    374 x 418   (17, 19)  52.0 -> 39.0 | 62.7 -> 51.5
+//    244 x 248  (61, 31)  39.8 -> 26.7 | 51.5 -> 41.1    510 x 512   (17)      45.2 -> 39.0 | 60.8 -> 61.4
+//    382 x 388  (191, 97) 60.0 -> 72.0 | 71.8 -> 83.5   1230 x 1230  (41)       207 -> 258  |  219 -> 279
 bool mixed_fft_eligible(int precision, int n1, int n2) {
-    MixedFft f;
-    auto side = [&](int n) { return n >= 64 && n <= kMixedMaxSide && factor(n, &f); };
+    auto side = [&](int n) {
+        MixedFft f;
+        return n >= 64 && n <= kMixedMaxSide && factor(n, &f) && (f.radix[0] <= 16 || 1LL * n1 * n2 <= 1 << 20);
+    };
     return precision == NFFT2D_F32 && side(n1) && side(n2);
 }
 
