@@ -490,10 +490,15 @@ struct TcGather {
 // direct and tensor cores, 2^22 / 2^20 / 400 k uniform points on 1024^2
 // coefficients (256 / 64 / 24 points a tile): w 8: 356 and 232 / 143 and 96 /
 // 81 and 83; w 7: 436 and 230 / 139 and 94 / 67 and 81; w 6: 270 and 214 / 114
-// and 90 / 59 and 79; w 5: 202 and 201 at 2^22.  Small sets give its
-// persistent CTAs too few batches: w 6, 2^18 points on 512^2, 32 and 35.
+// and 90 / 59 and 79; w 5: 202 and 201 at 2^22.  Clustered sets fill fewer of
+// its batches: w 6, 2^20 / 2^21 / 3 2^20 points (64 / 128 / 192 a tile), 87 and
+// 102 / 136 and 141 / 190 and 177; w 8, 64 a tile, 115 and 111.  So from 48
+// points a tile at w 7 and 8, and for a regridder's raster (whose tiles have no
+// strips), from 128 at w 6.  Small sets give its persistent CTAs too few
+// batches: w 6, 2^18 points on 512^2, 32 and 35.
 inline bool tc_gather_pays(int K, const Geom &g, long long M) {
-    return K >= 6 && g.T <= 16 && M >= (1LL << 19) && M >= 48LL * g.tiles1 * g.tiles2;
+    const long long per_tile = K > 6 || g.SW == g.T ? 48 : 128;
+    return K >= 6 && g.T <= 16 && M >= (1LL << 19) && M >= per_tile * g.tiles1 * g.tiles2;
 }
 
 }  // namespace nfft2d
