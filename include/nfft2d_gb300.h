@@ -110,16 +110,18 @@ typedef struct {
                               set_points from the bin density)                  */
     int spread_variant;    /* -1 = keep; NFFT2D_VARIANT_*                       */
     int compensated;       /* -1 = default (on); 0 off; 1 on (FP32 gather)      */
-    int fft_mode;          /* -1 = keep.  Initially automatic: 2 below 2048 x
-                              2048 oversampled cells where it applies, else 1
-                              from 2048 x 2048 cells up, else 0.
+    int fft_mode;          /* -1 = keep.  Initially automatic: fused passes
+                              (reported as 2) on sides that are powers of two
+                              below 2048 x 2048 oversampled cells and on other
+                              sides of small prime factors, else 1 from
+                              2048 x 2048 cells up, else 0.
                               0: one 2D cuFFT plan; 1: two 1D cuFFT passes, the
                               column pass only over the columns the band needs
                               (1.5 instead of 2 passes at sigma = 2); 2: the
                               library's own FFT passes fused with deapodize/pad,
-                              halo fill, halo fold and crop (FP32 plans, grid
-                              sides powers of two from 64 to 4096, else
-                              NFFT2D_ERR_UNSUPPORTED)                           */
+                              halo fill, halo fold and crop (FP32 plans; set
+                              here on grid sides that are powers of two from 64
+                              to 4096, else NFFT2D_ERR_UNSUPPORTED)             */
     int io_order;          /* -1 = keep.  NFFT2D_ORDER_CALLER (initially): the
                               per-point arrays (f of type 2 / type 1, v, g1,
                               g2 of grad_x) follow the caller's point order.

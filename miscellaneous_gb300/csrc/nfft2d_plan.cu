@@ -3,7 +3,9 @@
 // pad, halo fill/fold, crop+deapodize: used around cuFFT) and the C ABI entry
 // points of libnfft2d_gb300.so.  The oversampled FFT is the fused passes of
 // nfft2d_fft.cu for FP32 plans on power-of-two grids below 2048 x 2048 cells
-// (use_fused), cuFFT otherwise (run_fft).
+// (use_fused), those of nfft2d_fft_mixed.cu for sides of small prime factors
+// (use_mixed), cuFFT otherwise (run_fft); small transforms run in one launch
+// (use_small, nfft2d_small.cu).
 //
 // Reference path being replaced: NFFT/NFFT2_2D.cu:329-495 (NFFT2_2D_GPU:
 // constants, Kernel_Bessel, malloc/memset, Interpolation_NFFT2_2D_GPUKernel,

@@ -127,7 +127,8 @@ class Plan:
         gather_variant / spread_variant: _lib.VARIANT_AUTO, _TILED or _DIRECT.
         fft_mode: -1 keep, 0 cuFFT 2D plan, 1 cuFFT row/band-column passes,
         2 hand-written passes fused with pad/fill/fold/crop (FP32, power-of-two
-        grids; the default below 2048 x 2048 oversampled cells).
+        grids; the default below 2048 x 2048 oversampled cells, and with mixed
+        radices on other sides of small prime factors).
         io_order: None keep, 'caller' or 'binned' (per-point arrays in the
         plan's binned order, see permutation())."""
         io = -1 if io_order is None else {"caller": _lib.ORDER_CALLER, "binned": _lib.ORDER_BINNED}[io_order]
