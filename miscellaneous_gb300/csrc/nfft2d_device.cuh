@@ -88,6 +88,13 @@ __device__ __forceinline__ void bulk_wait_read_le1() {
 // Wait until every committed bulk group has completed (writes performed).
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Programmatic dependent launch.  start_next: the next kernel of the stream, if
+// launched with launch_after, may become resident once every CTA of this one
+// has come here.  wait_previous: until the kernels before have completed and
+// their writes are visible; returns at once in a kernel launched plainly.
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void latch_error(int *status, int bit) { atomicOr(status + 1, bit); }
 
 // ---------------------------------------------------------------------------

@@ -33,6 +33,9 @@
 // columns of consecutive rows), row passes keep them contiguous; shared
 // memory indices carry one pad element per 16.
 //
+// The second pass of a direction may start while the first ends (launch_after,
+// nfft2d_internal.h): its twiddles load meanwhile.
+//
 // The plan uses these passes by default below 2048 x 2048 oversampled cells
 // (nfft2d_plan.cu, use_fused).  From there up a row of 2048 or 4096 points
 // needs 128 or 256 threads at ~115 registers, two CTAs per SM, and cuFFT's
@@ -42,6 +45,7 @@
 #include <cmath>
 #include <vector>
 
+#include "nfft2d_device.cuh"
 #include "nfft2d_internal.h"
 
 namespace nfft2d {
@@ -263,6 +267,7 @@ __global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_cols_pad(const flo
                                                               const float *__restrict__ d2,
                                                               const float2 *__restrict__ tw, const FftArgs a) {
     extern __shared__ float2 fsm[];
+    start_next();
     Twiddles tws;
     prefetch_twiddles<true>(tws, a.logn1, a.logP, a.s, tw);
     const int P = 1 << a.logP, n1 = a.n1;
@@ -312,6 +317,8 @@ __global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_rows_fill(float2 *
     prefetch_twiddles<false>(tws, a.logn2, a.logP, a.s, tw);
     const int n2 = a.n2;
     const int r0 = blockIdx.x << a.logP;
+    start_next();
+    wait_previous();
     {
         float2 v[16];
 #pragma unroll
@@ -368,6 +375,8 @@ __global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_rows_fold(float2 *
     // CTAs holding edge rows look at row images
     float2 vs[16];
     const int H = a.H;
+    start_next();
+    wait_previous();
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
         const int e = threadIdx.x + u * blockDim.x;
@@ -406,7 +415,7 @@ __global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_rows_fold(float2 *
 
 // Type 1, pass 2: P band columns per CTA, transformed, cropped to the N1 band
 // rows and deapodized into F (N1 x N2, row-major).
-__global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_cols_crop(const float2 *__restrict__ grid, float2 *__restrict__ F,
+__global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_cols_crop(const float2 *grid, float2 *F,
                                                                const float *__restrict__ d1,
                                                                const float *__restrict__ d2,
                                                                const float2 *__restrict__ tw, const FftArgs a) {
@@ -415,6 +424,7 @@ __global__ void __launch_bounds__(kFftMaxElems / 16, 2) k_fft_cols_crop(const fl
     prefetch_twiddles<true>(tws, a.logn1, a.logP, a.s, tw);
     const int P = 1 << a.logP, n1 = a.n1;
     const int bc0 = blockIdx.x << a.logP;
+    wait_previous();
     {
         float2 v[16];
 #pragma unroll
@@ -544,8 +554,8 @@ cudaError_t fused_type2_rows(const nfft2d_plan_s *p, int sign) {
     const int smem = padded_elems(a.n2 << a.logP) * static_cast<int>(sizeof(float2));
     cudaError_t e = allow_smem(k_fft_rows_fill, smem);
     if (e != cudaSuccess) return e;
-    k_fft_rows_fill<<<blocks, threads, smem, p->stream>>>(static_cast<float2 *>(p->grid), p->tw2, a);
-    return cudaGetLastError();
+    return launch_after(k_fft_rows_fill, dim3(blocks), threads, smem, p->stream, static_cast<float2 *>(p->grid),
+                        static_cast<const float2 *>(p->tw2), a);
 }
 
 cudaError_t fused_type1_rows(const nfft2d_plan_s *p, int sign) {
@@ -556,8 +566,8 @@ cudaError_t fused_type1_rows(const nfft2d_plan_s *p, int sign) {
     const int smem = padded_elems(a.n2 << a.logP) * static_cast<int>(sizeof(float2));
     cudaError_t e = allow_smem(k_fft_rows_fold, smem);
     if (e != cudaSuccess) return e;
-    k_fft_rows_fold<<<blocks, threads, smem, p->stream>>>(static_cast<float2 *>(p->grid), p->tw2, a);
-    return cudaGetLastError();
+    return launch_after(k_fft_rows_fold, dim3(blocks), threads, smem, p->stream, static_cast<float2 *>(p->grid),
+                        static_cast<const float2 *>(p->tw2), a);
 }
 
 cudaError_t fused_type1_cols(const nfft2d_plan_s *p, int sign, void *F) {
@@ -568,10 +578,9 @@ cudaError_t fused_type1_cols(const nfft2d_plan_s *p, int sign, void *F) {
     const int smem = padded_elems(a.n1 << a.logP) * static_cast<int>(sizeof(float2));
     cudaError_t e = allow_smem(k_fft_cols_crop, smem);
     if (e != cudaSuccess) return e;
-    k_fft_cols_crop<<<blocks, threads, smem, p->stream>>>(
-        static_cast<const float2 *>(p->grid), static_cast<float2 *>(F), static_cast<const float *>(p->deap1),
-        static_cast<const float *>(p->deap2), p->tw1, a);
-    return cudaGetLastError();
+    return launch_after(k_fft_cols_crop, dim3(blocks), threads, smem, p->stream, static_cast<const float2 *>(p->grid),
+                        static_cast<float2 *>(F), static_cast<const float *>(p->deap1),
+                        static_cast<const float *>(p->deap2), static_cast<const float2 *>(p->tw1), a);
 }
 
 }  // namespace nfft2d

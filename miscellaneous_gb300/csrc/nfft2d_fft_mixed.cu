@@ -18,6 +18,7 @@
 
 #include <algorithm>
 
+#include "nfft2d_device.cuh"
 #include "nfft2d_internal.h"
 
 namespace nfft2d {
@@ -297,6 +298,7 @@ __global__ void __launch_bounds__(kMixedThreads) k_mixed_cols_pad(const float2 *
                                                                   const float2 *__restrict__ tw,
                                                                   const __grid_constant__ MixedArgs a) {
     extern __shared__ float2 sm[];
+    start_next();
     const int n1 = a.n1, N1 = a.N1, N2 = a.N2, bc0 = blockIdx.x << a.logP;
     float2 *const cell = grid + static_cast<size_t>(a.H) * a.C + a.H;
     mixed_fft(
@@ -319,6 +321,8 @@ __global__ void __launch_bounds__(kMixedThreads) k_mixed_cols_pad(const float2 *
 __global__ void __launch_bounds__(kMixedThreads) k_mixed_rows_fill(float2 *__restrict__ grid, const float2 *__restrict__ tw,
                                                                    const __grid_constant__ MixedArgs a) {
     extern __shared__ float2 sm[];
+    start_next();
+    wait_previous();
     const int n2 = a.n2, N2 = a.N2, r = blockIdx.x, H = a.H;
     float2 *const row = grid + static_cast<size_t>(r + H) * a.C + H;
     const ptrdiff_t dr = static_cast<ptrdiff_t>(r < H ? a.n1 : (r >= a.n1 - H ? -a.n1 : 0)) * a.C;
@@ -345,6 +349,8 @@ __global__ void __launch_bounds__(kMixedThreads) k_mixed_rows_fill(float2 *__res
 __global__ void __launch_bounds__(kMixedThreads) k_mixed_rows_fold(float2 *__restrict__ grid, const float2 *__restrict__ tw,
                                                                    const __grid_constant__ MixedArgs a) {
     extern __shared__ float2 sm[];
+    start_next();
+    wait_previous();
     const int n2 = a.n2, N2 = a.N2, r = blockIdx.x, H = a.H;
     float2 *const row = grid + static_cast<size_t>(r + H) * a.C + H;
     const ptrdiff_t dr = static_cast<ptrdiff_t>(r < H ? a.n1 : (r >= a.n1 - H ? -a.n1 : 0)) * a.C;
@@ -370,18 +376,19 @@ __global__ void __launch_bounds__(kMixedThreads) k_mixed_rows_fold(float2 *__res
 
 // Type 1, pass 2: P band columns a CTA, cropped to the N1 band rows and
 // deapodized into F.
-__global__ void __launch_bounds__(kMixedThreads) k_mixed_cols_crop(const float2 *__restrict__ grid, float2 *__restrict__ F,
+__global__ void __launch_bounds__(kMixedThreads) k_mixed_cols_crop(const float2 *grid, float2 *F,
                                                                    const float *__restrict__ d1,
                                                                    const float *__restrict__ d2,
                                                                    const float2 *__restrict__ tw,
                                                                    const __grid_constant__ MixedArgs a) {
     extern __shared__ float2 sm[];
+    wait_previous();
     const int n1 = a.n1, N1 = a.N1, N2 = a.N2, bc0 = blockIdx.x << a.logP;
     const float2 *const cell = grid + static_cast<size_t>(a.H) * a.C + a.H;
     mixed_fft(
         sm, a, tw,
         [&](int r, int q) {
-            return __ldg(cell + static_cast<size_t>(r) * a.C + band_col(min(bc0 + q, N2 - 1), N2, a.n2));
+            return __ldcg(cell + static_cast<size_t>(r) * a.C + band_col(min(bc0 + q, N2 - 1), N2, a.n2));
         },
         [&](int r, int q, float2 v) {
             const int k1 = r < n1 / 2 ? r : r - n1;
@@ -451,12 +458,13 @@ int block_threads(const Geom &g, int elems) {
 }
 
 template <typename Kernel, typename... Args>
-cudaError_t launch(Kernel kernel, const nfft2d_plan_s *p, int blocks, int elems, Args... args) {
+cudaError_t launch(Kernel kernel, const nfft2d_plan_s *p, bool after, int blocks, int elems, Args... args) {
     const int smem = 2 * padded(elems) * static_cast<int>(sizeof(float2)) + 16;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
+    if (after) return launch_after(kernel, dim3(blocks), block_threads(p->g, elems), smem, p->stream, args...);
     kernel<<<blocks, block_threads(p->g, elems), smem, p->stream>>>(args...);
     return cudaGetLastError();
 }
@@ -480,27 +488,27 @@ bool mixed_fft_eligible(int precision, int n1, int n2) {
 cudaError_t mixed_type2_cols(const nfft2d_plan_s *p, int sign, const void *F) {
     MixedArgs a = mixed_args(p, sign, p->g.n1);
     a.logP = cols_log(p);
-    return launch(k_mixed_cols_pad, p, (p->N2 + (1 << a.logP) - 1) >> a.logP, a.n1 << a.logP,
+    return launch(k_mixed_cols_pad, p, false, (p->N2 + (1 << a.logP) - 1) >> a.logP, a.n1 << a.logP,
                   static_cast<const float2 *>(F), static_cast<float2 *>(p->grid), static_cast<const float *>(p->deap1),
                   static_cast<const float *>(p->deap2), static_cast<const float2 *>(p->tw1), a);
 }
 
 cudaError_t mixed_type2_rows(const nfft2d_plan_s *p, int sign) {
     const MixedArgs a = mixed_args(p, sign, p->g.n2);
-    return launch(k_mixed_rows_fill, p, a.n1, a.n2, static_cast<float2 *>(p->grid),
+    return launch(k_mixed_rows_fill, p, true, a.n1, a.n2, static_cast<float2 *>(p->grid),
                   static_cast<const float2 *>(p->tw2), a);
 }
 
 cudaError_t mixed_type1_rows(const nfft2d_plan_s *p, int sign) {
     const MixedArgs a = mixed_args(p, sign, p->g.n2);
-    return launch(k_mixed_rows_fold, p, a.n1, a.n2, static_cast<float2 *>(p->grid),
+    return launch(k_mixed_rows_fold, p, true, a.n1, a.n2, static_cast<float2 *>(p->grid),
                   static_cast<const float2 *>(p->tw2), a);
 }
 
 cudaError_t mixed_type1_cols(const nfft2d_plan_s *p, int sign, void *F) {
     MixedArgs a = mixed_args(p, sign, p->g.n1);
     a.logP = cols_log(p);
-    return launch(k_mixed_cols_crop, p, (p->N2 + (1 << a.logP) - 1) >> a.logP, a.n1 << a.logP,
+    return launch(k_mixed_cols_crop, p, true, (p->N2 + (1 << a.logP) - 1) >> a.logP, a.n1 << a.logP,
                   static_cast<const float2 *>(p->grid), static_cast<float2 *>(F), static_cast<const float *>(p->deap1),
                   static_cast<const float *>(p->deap2), static_cast<const float2 *>(p->tw1), a);
 }

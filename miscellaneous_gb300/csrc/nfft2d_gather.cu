@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? 4 : 2) k_gather_tiled(co
         fence_proxy_async_smem();
     }
     __syncthreads();  // the only CTA-wide barrier: the mbarriers are initialised
+    wait_previous();  // the grid, which only TMA loads read, is complete
     if (threadIdx.x == 0 && static_cast<int>(blockIdx.x) < n) issue_patch<K>(&tmap, chunks, blockIdx.x, bufs, &full[0], g);
 
     int it = 0;
@@ -362,10 +363,10 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
         if (e != cudaSuccess) return e;
         int blocks = grid_blocks(p, reinterpret_cast<const void *>(kernel), kThreads, smem);
         if (p->n_chunks >= 0 && blocks > p->n_chunks) blocks = static_cast<int>(p->n_chunks);
-        kernel<<<blocks, kThreads, smem, p->stream>>>(p->tmap, static_cast<const Rec32 *>(p->recs), p->chunks,
-                                                      static_cast<float2 *>(f), static_cast<const float2 *>(v),
-                                                      static_cast<float *>(g1), static_cast<float *>(g2), a);
-        return cudaGetLastError();
+        return launch_after(kernel, dim3(blocks), kThreads, smem, p->stream, p->tmap,
+                            static_cast<const Rec32 *>(p->recs), static_cast<const int4 *>(p->chunks),
+                            static_cast<float2 *>(f), static_cast<const float2 *>(v), static_cast<float *>(g1),
+                            static_cast<float *>(g2), a);
     }
     const int blocks = static_cast<int>((p->M + kThreads - 1) / kThreads);
     if (blocks == 0) return cudaSuccess;

@@ -774,6 +774,7 @@ __global__ void k_bin_pass1(const CT *__restrict__ x1, const CT *__restrict__ x2
                             int *__restrict__ status, unsigned long long *__restrict__ scan_state,
                             int scan_words) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    start_next();
     // the two scans that follow start from zeroed tickets and tile words
     for (int k = i; k < scan_words; k += gridDim.x * blockDim.x) scan_state[k] = 0ull;
     if (i >= M) return;
@@ -801,9 +802,10 @@ __global__ void k_bin_pass1(const CT *__restrict__ x1, const CT *__restrict__ x2
 // = i.  The 4-byte writes land in an array a quarter of the records' size,
 // which stays in L2 where the writes merge into whole lines.
 template <bool STREAM>
-__global__ void k_bin_invert(const uint2 *__restrict__ keyrank, const unsigned *__restrict__ cell_start, int M,
-                             int *__restrict__ src) {
+__global__ void k_bin_invert(const uint2 *keyrank, const unsigned *cell_start, int M, int *src) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    start_next();
+    wait_previous();
     if (i >= M) return;
     const uint2 kr = ld_once<STREAM>(keyrank + i);
     src[cell_start[kr.x] + kr.y] = i;
@@ -813,9 +815,10 @@ __global__ void k_bin_invert(const uint2 *__restrict__ keyrank, const unsigned *
 // random reads and coalesced writes (a scatter of the 16-byte records would
 // write half sectors at random addresses of an array larger than L2).
 template <typename RecT, bool STREAM>
-__global__ void k_bin_gather(const RecT *__restrict__ tmp, const int *__restrict__ src, int M,
-                             RecT *__restrict__ recs) {
+__global__ void k_bin_gather(const RecT *tmp, const int *src, int M, RecT *recs) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    start_next();
+    wait_previous();
     if (q >= M) return;
     st_rec<STREAM>(recs + q, tmp[ld_once<STREAM>(src + q)]);
 }
@@ -1186,9 +1189,11 @@ __device__ __forceinline__ int scan_ticket(unsigned long long *state) {
 }
 
 // In-place exclusive scan of n counters.
-__global__ void __launch_bounds__(kCellScanThreads) k_scan_counts(unsigned *__restrict__ data, size_t n,
+__global__ void __launch_bounds__(kCellScanThreads) k_scan_counts(unsigned *data, size_t n,
                                                                   unsigned long long *state, int *status) {
     constexpr int ITEMS = kCellScanItems;
+    start_next();
+    wait_previous();
     const int tile = scan_ticket(state);
     const size_t base = static_cast<size_t>(tile) * (kCellScanThreads * ITEMS) +
                         static_cast<size_t>(threadIdx.x) * ITEMS;
@@ -1222,12 +1227,14 @@ __global__ void __launch_bounds__(kCellScanThreads) k_scan_counts(unsigned *__re
 // t * cells_per_tile) holds ceil(count / chunk) items of up to `chunk`
 // points.  One scan over the per-tile item counts places every tile's items;
 // the thread owning index ntiles stores the total in *total.
-__global__ void __launch_bounds__(kItemScanThreads, 1) k_scan_emit_chunks(const unsigned *__restrict__ cell_start,
+__global__ void __launch_bounds__(kItemScanThreads, 1) k_scan_emit_chunks(const unsigned *cell_start,
                                                                        int ntiles, int cells_per_tile, int chunk,
                                                                        int4 *__restrict__ chunks,
                                                                        unsigned long long *state, int *status,
                                                                        int *total) {
     static_assert(kItemScanItems == 1, "one bin tile per thread");
+    start_next();
+    wait_previous();
     const int tile = scan_ticket(state);
     const long long t = static_cast<long long>(tile) * kItemScanThreads + threadIdx.x;  // bin tile
     unsigned start = 0, cnt = 0;
@@ -2170,14 +2177,15 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
             if (e != cudaSuccess) return e;
             if (coords_read && (e = cudaEventRecord(coords_read, p->stream)) != cudaSuccess) return e;  // coordinates read
             const size_t cells_n = p->ncells + 1;
-            k_scan_counts<<<static_cast<unsigned>((cells_n + kCellTile - 1) / kCellTile), kCellScanThreads, 0,
-                            p->stream>>>(p->cell_count, cells_n, scan_state, p->d_status);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            k_bin_invert<S><<<blocks, 256, 0, p->stream>>>(p->keyrank, p->cell_count, Mi, p->src);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            k_bin_gather<RecT, S><<<blocks, 256, 0, p->stream>>>(static_cast<const RecT *>(p->tmp_recs), p->src, Mi,
-                                                                  static_cast<RecT *>(p->recs));
-            return cudaGetLastError();
+            e = launch_after(k_scan_counts, dim3(static_cast<unsigned>((cells_n + kCellTile - 1) / kCellTile)),
+                             kCellScanThreads, 0, p->stream, p->cell_count, cells_n, scan_state, p->d_status);
+            if (e != cudaSuccess) return e;
+            e = launch_after(k_bin_invert<S>, dim3(blocks), 256, 0, p->stream, static_cast<const uint2 *>(p->keyrank),
+                             static_cast<const unsigned *>(p->cell_count), Mi, p->src);
+            if (e != cudaSuccess) return e;
+            return launch_after(k_bin_gather<RecT, S>, dim3(blocks), 256, 0, p->stream,
+                                static_cast<const RecT *>(p->tmp_recs), static_cast<const int *>(p->src), Mi,
+                                static_cast<RecT *>(p->recs));
         };
         using Yes = std::true_type;
         using No = std::false_type;
@@ -2198,14 +2206,13 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
         const int ntiles = g.tiles1 * g.tiles2;
         const unsigned emit_blocks = static_cast<unsigned>((ntiles + 1 + kItemTile - 1) / kItemTile);
         unsigned long long *item_state = scan_state + scan_state_words(cells_n, kCellTile);
-        k_scan_emit_chunks<<<emit_blocks, kItemScanThreads, 0, p->stream>>>(
-            p->cell_count, ntiles, g.T * g.T, p->chunk, p->chunks, item_state, p->d_status, p->d_status);
-        NFFT_TRY_CUDA(cudaGetLastError());
+        NFFT_TRY_CUDA(launch_after(k_scan_emit_chunks, dim3(emit_blocks), kItemScanThreads, 0, p->stream,
+                                   static_cast<const unsigned *>(p->cell_count), ntiles, g.T * g.T, p->chunk, p->chunks,
+                                   item_state, p->d_status, p->d_status));
         if (p->chunk > kSpreadItemMax) {  // the spread's own work list, count in status[3]
-            k_scan_emit_chunks<<<emit_blocks, kItemScanThreads, 0, p->stream>>>(
-                p->cell_count, ntiles, g.T * g.T, kSpreadItemMax, p->items, item_state + item_words, p->d_status,
-                p->d_status + 3);
-            NFFT_TRY_CUDA(cudaGetLastError());
+            NFFT_TRY_CUDA(launch_after(k_scan_emit_chunks, dim3(emit_blocks), kItemScanThreads, 0, p->stream,
+                                       static_cast<const unsigned *>(p->cell_count), ntiles, g.T * g.T, kSpreadItemMax,
+                                       p->items, item_state + item_words, p->d_status, p->d_status + 3));
         }
     }
     stage_end(p, ST_SORT);

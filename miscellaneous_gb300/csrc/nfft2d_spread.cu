@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_tiled(const __grid
                                                                     const float2 *__restrict__ f,
                                                                     const __grid_constant__ KArgs a) {
     extern __shared__ unsigned char smem_raw[];
+    start_next();
     using S = SpreadGeo<K>;
     const Geom g = a.g;  // g.T == kRegTile, g.SW == S::SW
     // TMA shared-memory operands: 128-byte aligned (the launch adds 128 bytes of slack)
