@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kThreads64) k_gather_direct_f64(const double2 
 // uniform 67.5 -> 61.3 us at K = 6).
 template <int K>
 __global__ void __launch_bounds__(kThreads, K <= 6 ? 4 : 3)
-    k_gather_direct_f32(const float2 *__restrict__ grid, const Rec32 *__restrict__ recs, float2 *__restrict__ out,
+    k_gather_direct_f32(const float2 *grid, const Rec32 *__restrict__ recs, float2 *out,
                         const __grid_constant__ KArgs a) {
     const int i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= a.M) return;
@@ -250,11 +250,13 @@ __global__ void __launch_bounds__(kThreads, K <= 6 ? 4 : 3)
     const int mu1 = static_cast<int>(static_cast<unsigned>(r.mu) >> 16), mu2 = r.mu & 0xFFFF;
     const Geom g = a.g;
     if (mu1 >= g.n1 || mu2 >= g.n2) {
+        wait_previous();
         latch_error(a.status, kErrBounds);
         return;
     }
-    out[a.binned_io ? i : r.orig] = a.compensated ? gather_direct_f32<K, true>(grid, g.H, g.C, mu1, mu2, r.t1, r.t2, a.poly)
-                                : gather_direct_f32<K, false>(grid, g.H, g.C, mu1, mu2, r.t1, r.t2, a.poly);
+    out[a.binned_io ? i : r.orig] = a.compensated
+                                        ? gather_direct_f32<K, true, true>(grid, g.H, g.C, mu1, mu2, r.t1, r.t2, a.poly)
+                                        : gather_direct_f32<K, false, true>(grid, g.H, g.C, mu1, mu2, r.t1, r.t2, a.poly);
 }
 
 // The direct gather's results from the tensor cores (nfft2d_tc.cuh), for
@@ -388,8 +390,9 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
                 return cudaGetLastError();
             }
         }
-        k_gather_direct_f32<K><<<blocks, kThreads, 0, p->stream>>>(
-            static_cast<const float2 *>(p->grid), static_cast<const Rec32 *>(p->recs), static_cast<float2 *>(f), a);
+        return launch_after(k_gather_direct_f32<K>, dim3(blocks), kThreads, 0, p->stream,
+                            static_cast<const float2 *>(p->grid), static_cast<const Rec32 *>(p->recs),
+                            static_cast<float2 *>(f), a);
     } else {
         static_assert(MODE == 0 || MODE == 1, "gather (0) or coordinate gradient (1)");
         k_grad_direct_f32<K><<<blocks, kThreads, 0, p->stream>>>(

@@ -1548,6 +1548,23 @@ int grid_blocks(const nfft2d_plan_s *p, const void *kernel, int threads, int sme
     return per_sm * std::max(1, p->num_sms);
 }
 
+// The grid and the spread's work counter to zero, in a kernel, so that the
+// spread may start while it ends: two fills before the spread cost it 3 us.
+__global__ void k_zero_grid(float4 *grid, size_t n, int *work) {
+    start_next();
+    const size_t i0 = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+    if (i0 == 0) *work = 0;
+    for (size_t i = i0; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) grid[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+cudaError_t launch_zero_grid(const nfft2d_plan_s *p) {
+    // rows of an even number of cells: whole 16 bytes
+    const size_t n = cplx_size(p->precision) * static_cast<size_t>(p->g.Ra) * p->g.C / sizeof(float4);
+    const size_t blocks = std::min<size_t>((n + 255) / 256, 16u * static_cast<size_t>(p->num_sms));
+    k_zero_grid<<<static_cast<unsigned>(blocks), 256, 0, p->stream>>>(static_cast<float4 *>(p->grid), n, p->d_status + 2);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pad(const nfft2d_plan_s *p, const void *F) {
     const Geom &g = p->g;
     const dim3 grid = row_grid(g.n2, g.n1);
@@ -2301,7 +2318,7 @@ static int nfft2d_type1_impl(nfft2d_plan p, int sign, const void *f, void *F) {
         return NFFT2D_OK;
     }
     stage_begin(p, ST_SPREAD);
-    NFFT_TRY_CUDA(cudaMemsetAsync(p->grid, 0, cplx_size(p->precision) * static_cast<size_t>(g.Ra) * g.C, p->stream));
+    NFFT_TRY_CUDA(launch_zero_grid(p));
     NFFT_TRY_CUDA(launch_spread(p, f));
     stage_end(p, ST_SPREAD);
     if (use_fused(p) || use_mixed(p)) {  // fold + row FFT, then band-column FFT + crop

@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kSpreadWarps * 32) k_spread_tiled(const __grid
     int *work = a.status + 2;  // work-item counter, zeroed before the launch
     StripFlush fs{&tmap, bufs, g.H, 0};
     strip_flush_init<K>(fs, scr);
+    wait_previous();  // the grid and the work counter are zero
 
     // A warp's work item is one whole entry of the work list: the plan's
     // chunks (up to `chunk` points of one tile), or for chunks above
@@ -137,8 +138,6 @@ cudaError_t launch_K(const nfft2d_plan_s *p, const void *f) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
         }
-        cudaError_t e = cudaMemsetAsync(p->d_status + 2, 0, sizeof(int), p->stream);
-        if (e != cudaSuccess) return e;
         int blocks = grid_blocks(p, reinterpret_cast<const void *>(kernel), kSpreadWarps * 32, smem);
         const bool own_list = p->chunk > kSpreadItemMax;  // its count stays on the device (status[3])
         const int n_host = own_list ? -1 : static_cast<int>(p->n_chunks);
@@ -146,10 +145,10 @@ cudaError_t launch_K(const nfft2d_plan_s *p, const void *f) {
             const int need = (n_host + kSpreadWarps - 1) / kSpreadWarps;
             if (blocks > need) blocks = need;
         }
-        kernel<<<blocks, kSpreadWarps * 32, smem, p->stream>>>(
-            p->tmap_spread, static_cast<const Rec32 *>(p->recs), own_list ? p->items : p->chunks, n_host,
-            p->d_status + (own_list ? 3 : 0), static_cast<const float2 *>(f), a);
-        return cudaGetLastError();
+        return launch_after(kernel, dim3(blocks), kSpreadWarps * 32, smem, p->stream, p->tmap_spread,
+                            static_cast<const Rec32 *>(p->recs),
+                            static_cast<const int4 *>(own_list ? p->items : p->chunks), n_host,
+                            static_cast<const int *>(p->d_status + (own_list ? 3 : 0)), static_cast<const float2 *>(f), a);
     }
     const int blocks = static_cast<int>((p->M + kThreads - 1) / kThreads);
     if (blocks == 0) return cudaSuccess;

@@ -63,9 +63,10 @@ __device__ __forceinline__ float2 gather_point(const float2 *__restrict__ patch,
 //
 // COMP: the weighted row partials are summed with TwoSum and the rounding
 // errors carried in a second accumulator (as the tiled gather does), else
-// with plain FMAs.
-template <int K, bool COMP>
-__device__ __forceinline__ float2 gather_direct_f32(const float2 *__restrict__ grid, int H, int C, int mu1, int mu2,
+// with plain FMAs.  WAIT: the grid is the kernel before's, complete once the
+// weights are formed (so it is read by plain loads, not the read-only path).
+template <int K, bool COMP, bool WAIT = false>
+__device__ __forceinline__ float2 gather_direct_f32(const float2 *grid, int H, int C, int mu1, int mu2,
                                                     float t1, float t2, const WinPoly &wp) {
     constexpr int W = 2 * K + 1;
     constexpr int V = K + 1;  // float4 loads per row
@@ -87,6 +88,7 @@ __device__ __forceinline__ float2 gather_direct_f32(const float2 *__restrict__ g
     float2 wsp[2 * V];
 #pragma unroll
     for (int q = 0; q < 2 * V; ++q) wsp[q] = make_float2(ws[q], ws[q]);
+    if constexpr (WAIT) wait_previous();
     float2 s = make_float2(0.f, 0.f), e = make_float2(0.f, 0.f);
 #pragma unroll
     for (int rr = 0; rr < W; ++rr) {
@@ -94,7 +96,7 @@ __device__ __forceinline__ float2 gather_direct_f32(const float2 *__restrict__ g
         float2 r = make_float2(0.f, 0.f);
 #pragma unroll
         for (int q = 0; q < V; ++q) {
-            const float4 v = __ldg(row + q);
+            const float4 v = WAIT ? row[q] : __ldg(row + q);
             r = __ffma2_rn(make_float2(v.x, v.y), wsp[2 * q], r);
             r = __ffma2_rn(make_float2(v.z, v.w), wsp[2 * q + 1], r);
         }
