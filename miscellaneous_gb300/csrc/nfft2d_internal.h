@@ -309,10 +309,10 @@ void plan_free(void *ptr);
 // kernel calls wait_previous() before it touches what that one wrote, and reads
 // that by plain loads or TMA, never by the read-only path, whose lines may be
 // older than the wait.  For the short chains: cell scan to work items, column
-// to row pass to tiled gather, spread to fold to crop.  The gap between two
+// to row pass to gather, zeroing to spread to fold to crop.  The gap between two
 // dependent kernels is 1 to 2 us of launch and ramp.  Measured on GB300, us:
-// 256^2 coefficients, 9 k points, both directions 55.3 -> 50.3; 250 x 378, 300
-// k 80.9 -> 78.6; binning 2^20 points and transforming them 152 -> 142.
+// 256^2 coefficients, 9 k points, both directions 55.3 -> 47.2; 250 x 378, 300
+// k 80.9 -> 72.0; binning 2^20 points and transforming them 152 -> 142.
 template <typename Kernel, typename... Args>
 cudaError_t launch_after(Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream, Args... args) {
     cudaLaunchAttribute at;

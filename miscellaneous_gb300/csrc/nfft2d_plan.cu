@@ -395,20 +395,21 @@ bool use_mixed(const nfft2d_plan_s *p) {
 // grids, where launches and latency are most of the time: with the plan's own
 // choice of stages, and no stage to time.  Measured on GB300, one launch
 // against the separate kernels, w 6, us (forward | adjoint):
-//    64^2 coefficients   4096 points  15.2 / 19.6 | 16.5 / 34.9
-//    64^2               16000         19.6 / 21.6 | 24.8 / 44.6
-//   128^2                4096         18.5 / 20.5 | 22.6 / 32.5
-//   128^2               16000         20.6 / 20.6 | 28.7 / 37.1
-//   128^2               30000         24.6 / 22.6 | 34.5 / 39.1
-//   256^2                8000         30.8 / 22.6 | 38.0 / 35.1
-// so up to 256^2 cells, with 2^13 points forward (2^14 on 128^2 cells) and
-// 2^15 points adjoint.
+//    64^2 coefficients   4096 points  14.7 / 14.4 | 16.5 / 25.7
+//    64^2               16000         20.0 / 16.4 | 24.7 / 34.9
+//    64^2               32000              -      | 30.8 / 33.4
+//   128^2                4096         18.5 / 14.4 | 22.6 / 24.6
+//   128^2                8000              -      | 24.6 / 24.7
+//   128^2               16000         16.4 / 16.4 | 28.7 / 26.7
+// and forward and adjoint in turn at 64^2, 4096 points: 31.1 with both in one
+// launch each, 34.0 with the adjoint only.  So up to 128^2 cells, 2^13 points
+// forward and 2^15 adjoint; on more cells adjoints of up to 2^12 points.
 bool use_small(const nfft2d_plan_s *p, bool adjoint) {
     if (!p->small_ok || !p->gather_auto || p->spread_variant != NFFT2D_VARIANT_TILED || p->fft_mode >= 0 ||
         p->timer.on || p->g.T != 16 || p->g.SW != spread_strip_width(p->K) || p->chunk > kSpreadItemMax)
         return false;
-    const long long cells = 1LL * p->g.n1 * p->g.n2;
-    return p->M <= (adjoint ? 1 << 15 : cells <= 128 * 128 ? 1 << 14 : 1 << 13);
+    if (1LL * p->g.n1 * p->g.n2 > 128 * 128) return adjoint && p->M <= 1 << 12;
+    return p->M <= (adjoint ? 1 << 15 : 1 << 13);
 }
 
 // The automatic FP32 gather: the direct 16-byte-load gather from 128 points
