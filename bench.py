@@ -1142,11 +1142,11 @@ def run_ours(args, wl):
             "precision_study": study,
             "binned_io": binned,
             "spread_small_cases": small,
-            "gpu_launches": 6 * args.steps,
+            "gpu_launches": 7 * args.steps,
             "gpu_launches_note": ("our kernels in the timed region per step: column FFT+pad, row FFT+fill, gather, "
-                                  "spread, fold+row FFT, column FFT+crop") if fused else
-                                 ("our kernels in the timed region per step: pad, halo_fill, gather, spread, fold, "
-                                  "crop (cuFFT kernels not counted)"),
+                                  "grid zeroing, spread, fold+row FFT, column FFT+crop") if fused else
+                                 ("our kernels in the timed region per step: pad, halo_fill, gather, grid zeroing, "
+                                  "spread, fold, crop (cuFFT kernels not counted)"),
             "clocks": clocks.summary(),
         }
         print(json.dumps(line))
