@@ -351,7 +351,7 @@ cudaError_t prepare_smem(KernelT kernel, int smem) {
 }
 
 template <int K, int MODE>
-cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, void *g2) {
+cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, void *g2, bool after) {
     const KArgs a = make_kargs(p);
     if (p->precision == NFFT2D_F32 && p->gather_variant == NFFT2D_VARIANT_TILED) {
         if (p->n_chunks == 0) return cudaSuccess;
@@ -365,10 +365,10 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
         if (e != cudaSuccess) return e;
         int blocks = grid_blocks(p, reinterpret_cast<const void *>(kernel), kThreads, smem);
         if (p->n_chunks >= 0 && blocks > p->n_chunks) blocks = static_cast<int>(p->n_chunks);
-        return launch_after(kernel, dim3(blocks), kThreads, smem, p->stream, p->tmap,
-                            static_cast<const Rec32 *>(p->recs), static_cast<const int4 *>(p->chunks),
-                            static_cast<float2 *>(f), static_cast<const float2 *>(v), static_cast<float *>(g1),
-                            static_cast<float *>(g2), a);
+        return launch_chained(after, kernel, dim3(blocks), kThreads, smem, p->stream, p->tmap,
+                              static_cast<const Rec32 *>(p->recs), static_cast<const int4 *>(p->chunks),
+                              static_cast<float2 *>(f), static_cast<const float2 *>(v), static_cast<float *>(g1),
+                              static_cast<float *>(g2), a);
     }
     const int blocks = static_cast<int>((p->M + kThreads - 1) / kThreads);
     if (blocks == 0) return cudaSuccess;
@@ -390,9 +390,9 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
                 return cudaGetLastError();
             }
         }
-        return launch_after(k_gather_direct_f32<K>, dim3(blocks), kThreads, 0, p->stream,
-                            static_cast<const float2 *>(p->grid), static_cast<const Rec32 *>(p->recs),
-                            static_cast<float2 *>(f), a);
+        return launch_chained(after, k_gather_direct_f32<K>, dim3(blocks), kThreads, 0, p->stream,
+                              static_cast<const float2 *>(p->grid), static_cast<const Rec32 *>(p->recs),
+                              static_cast<float2 *>(f), a);
     } else {
         static_assert(MODE == 0 || MODE == 1, "gather (0) or coordinate gradient (1)");
         k_grad_direct_f32<K><<<blocks, kThreads, 0, p->stream>>>(
@@ -403,25 +403,27 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
 }
 
 template <int MODE>
-cudaError_t dispatch(const nfft2d_plan_s *p, void *f, const void *v, void *g1, void *g2) {
+cudaError_t dispatch(const nfft2d_plan_s *p, void *f, const void *v, void *g1, void *g2, bool after) {
     switch (p->K) {
-        case 2: return launch_K<2, MODE>(p, f, v, g1, g2);
-        case 3: return launch_K<3, MODE>(p, f, v, g1, g2);
-        case 4: return launch_K<4, MODE>(p, f, v, g1, g2);
-        case 5: return launch_K<5, MODE>(p, f, v, g1, g2);
-        case 6: return launch_K<6, MODE>(p, f, v, g1, g2);
-        case 7: return launch_K<7, MODE>(p, f, v, g1, g2);
-        case 8: return launch_K<8, MODE>(p, f, v, g1, g2);
+        case 2: return launch_K<2, MODE>(p, f, v, g1, g2, after);
+        case 3: return launch_K<3, MODE>(p, f, v, g1, g2, after);
+        case 4: return launch_K<4, MODE>(p, f, v, g1, g2, after);
+        case 5: return launch_K<5, MODE>(p, f, v, g1, g2, after);
+        case 6: return launch_K<6, MODE>(p, f, v, g1, g2, after);
+        case 7: return launch_K<7, MODE>(p, f, v, g1, g2, after);
+        case 8: return launch_K<8, MODE>(p, f, v, g1, g2, after);
         default: return cudaErrorInvalidValue;
     }
 }
 
 }  // namespace
 
-cudaError_t launch_gather(const nfft2d_plan_s *p, void *f) { return dispatch<0>(p, f, nullptr, nullptr, nullptr); }
+cudaError_t launch_gather(const nfft2d_plan_s *p, void *f, bool after) {
+    return dispatch<0>(p, f, nullptr, nullptr, nullptr, after);
+}
 
 cudaError_t launch_grad(const nfft2d_plan_s *p, const void *v, void *g1, void *g2) {
-    return dispatch<1>(p, nullptr, v, g1, g2);
+    return dispatch<1>(p, nullptr, v, g1, g2, true);
 }
 
 int gather_smem_bytes(const nfft2d_plan_s *p) { return 2 * patch_stride_elems(p->g) * static_cast<int>(sizeof(float2)) + 128; }

@@ -197,7 +197,9 @@ cudaError_t launch_halo_fill(const nfft2d_plan_s *p);
 cudaError_t launch_halo_fold(const nfft2d_plan_s *p);
 
 // gather.cu
-cudaError_t launch_gather(const nfft2d_plan_s *p, void *f);
+// after: the gather may begin while the kernel before it in the stream ends
+// (launch_after); false where that kernel belongs to the binning.
+cudaError_t launch_gather(const nfft2d_plan_s *p, void *f, bool after = true);
 cudaError_t launch_grad(const nfft2d_plan_s *p, const void *v, void *g1, void *g2);
 int gather_smem_bytes(const nfft2d_plan_s *p);
 
@@ -308,13 +310,19 @@ void plan_free(void *ptr);
 // A launch that may begin while the kernel before it in the stream ends; the
 // kernel calls wait_previous() before it touches what that one wrote, and reads
 // that by plain loads or TMA, never by the read-only path, whose lines may be
-// older than the wait.  For the short chains: cell scan to work items, column
+// older than the wait.  Of this kernel's ancestors the wait covers all, but what
+// it reads before the wait must have been complete when the last kernel launched
+// plainly on this stream began: so the gather, which loads its records and work
+// items first, is launched plainly where the binning precedes it directly
+// (bin_and_forward: the padding and the FFT are on another stream).
+// For the short chains: cell scan to work items, column
 // to row pass to gather, zeroing to spread to fold to crop.  The gap between two
 // dependent kernels is 1 to 2 us of launch and ramp.  Measured on GB300, us:
 // 256^2 coefficients, 9 k points, both directions 55.3 -> 47.2; 250 x 378, 300
 // k 80.9 -> 72.0; binning 2^20 points and transforming them 152 -> 142.
 template <typename Kernel, typename... Args>
-cudaError_t launch_after(Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_chained(bool after, Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream,
+                           Args... args) {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -324,8 +332,12 @@ cudaError_t launch_after(Kernel kernel, dim3 grid, int threads, int smem, cudaSt
     cfg.dynamicSmemBytes = static_cast<size_t>(smem);
     cfg.stream = stream;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = after ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename Kernel, typename... Args>
+cudaError_t launch_after(Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream, Args... args) {
+    return launch_chained(true, kernel, grid, threads, smem, stream, args...);
 }
 
 // The fused FFT passes (nfft2d_fft.cu): eligibility, per-plan twiddle tables,

@@ -2435,7 +2435,7 @@ int nfft2d_bin_and_forward(nfft2d_plan p, long long M, const void *x1, const voi
     NFFT_TRY_CUDA(cudaStreamWaitEvent(main, p->ev_join, 0));
     if (M == 0) return NFFT2D_OK;
     stage_begin(p, ST_GATHER);
-    NFFT_TRY_CUDA(launch_gather(p, f));
+    NFFT_TRY_CUDA(launch_gather(p, f, false));  // the kernels before it on this stream are the binning's
     stage_end(p, ST_GATHER);
     return NFFT2D_OK;
 }
