@@ -253,6 +253,11 @@ int nfft2d_selftest_wait_timeout(int spin_limit, void *stream);
  * the plan's status word as the plan's own kernels do: the next
  * nfft2d_synchronize returns NFFT2D_ERR_DEVICE_TIMEOUT (once).  Asynchronous. */
 int nfft2d_plan_selftest_wait_timeout(nfft2d_plan plan, int spin_limit);
+/* The plan's one-launch binning and transforms give up at their grid barrier
+ * `barrier` (1 to 3) from the next call on, as they do when a wait runs out;
+ * 0 ends that.  The next nfft2d_synchronize reports
+ * NFFT2D_ERR_DEVICE_TIMEOUT.  Host only. */
+int nfft2d_plan_selftest_barrier(nfft2d_plan plan, int barrier);
 
 /* ---- exact direct sum ----------------------------------------------------
  * Matrix-free FP64 replacement of NDFT2_2D_GPU (NFFT/NDFT2_2D.cu:37-72):

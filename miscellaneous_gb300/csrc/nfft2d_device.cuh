@@ -101,40 +101,49 @@ __device__ __forceinline__ void latch_error(int *status, int bit) { atomicOr(sta
 // barrier of a cooperative grid of kGridCtas CTAs (all resident: one an SM)
 // ---------------------------------------------------------------------------
 constexpr int kGridCtas = 128;
-// What any CTA wrote before it arrived, every thread of the kernel sees after
-// the wait; `target`: the CTAs' arrivals so far.  False, latched, if the wait
-// runs out (the CTA leaves; so do the others, by their own waits).
+// What any CTA wrote before it arrived at a barrier (1, 2, ...), every thread of
+// the kernel sees after the wait.  False, latched, if the wait runs out: the CTA
+// leaves, by grid_done as on every way out, and so do the others, by their own
+// waits.  give_up: the barrier whose waits all run out at once (self-test), or 0.
 __device__ __forceinline__ void grid_arrive(int *status) {
     __syncthreads();
     if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(status + kBarrierWord) : "memory");
 }
-__device__ __forceinline__ bool grid_wait(int *status, int target) {
+__device__ __forceinline__ bool grid_wait(int *status, int barrier, int give_up) {
     __shared__ int ok;
     if (threadIdx.x == 0) {
+        const int target = barrier * kGridCtas;
         int seen = 0;
         uint32_t spins = 0;
         do
             asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(status + kBarrierWord) : "memory");
-        while (seen < target && ++spins < kSpinLimit);
-        ok = seen >= target;
+        while (seen < target && ++spins < kSpinLimit && barrier != give_up);
+        ok = seen >= target && barrier != give_up;
         if (!ok) latch_error(status, kErrTimeout);
     }
     __syncthreads();
     return ok != 0;
 }
-__device__ __forceinline__ bool grid_barrier(int *status, int target) {
+__device__ __forceinline__ bool grid_barrier(int *status, int barrier, int give_up) {
     grid_arrive(status);
-    return grid_wait(status, target);
+    return grid_wait(status, barrier, give_up);
 }
-// The last CTA to come here leaves the barrier's words zero for the next launch.
-__device__ __forceinline__ void grid_done(int *status) {
+// The last CTA to come here leaves the barrier's words zero for the next launch,
+// whether or not a wait has run out: every CTA ends with this, and none arrives
+// at a barrier after it.  `failed`: a wait of this CTA has run out.  True in one
+// thread of the last CTA, if any has; what a failed CTA wrote, and what others
+// wrote before they arrived at a barrier, is in memory by then.
+__device__ __forceinline__ bool grid_done(int *status, bool failed) {
+    constexpr int kFailed = 1 << 16;
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(status + kBarrierWord + 1, 1) == kGridCtas - 1) {
-        status[kBarrierWord] = 0;
-        status[kBarrierWord + 1] = 0;
-    }
+    if (threadIdx.x != 0) return false;
+    if (failed) __threadfence();
+    const int sum = atomicAdd(status + kBarrierWord + 1, failed ? kFailed + 1 : 1) + (failed ? kFailed + 1 : 1);
+    if ((sum & (kFailed - 1)) != kGridCtas) return false;
+    status[kBarrierWord] = 0;
+    status[kBarrierWord + 1] = 0;
+    return sum >= kFailed;
 }
-
 
 // ---------------------------------------------------------------------------
 // Window pair.  The reference window (NFFT1_2D.m:34-36, NFFT2_2D.cu:112-122)

@@ -22,7 +22,7 @@ constexpr int kErrNonfinite = 4;
 
 // d_status: [0] work items, [1] error bits, [2] the spread's work counter, [3]
 // its own work items, [4] [5] the grid barrier of the one-launch transforms
-// (zero between launches).
+// (zero between launches, those that give up included).
 constexpr int kStatusWords = 6, kBarrierWord = 4;
 
 // One binned point, FP32 plans: fractional offsets t = sigma*x_grid - mu in
@@ -177,6 +177,7 @@ struct nfft2d_plan_s {
     bool fused_ok = false;                   // twiddle tables of the fused passes are set up
     bool mixed_ok = false;                   // as fused_ok, for sides of small prime factors
     bool small_ok = false;                   // the one-launch transforms fit the plan and the device
+    int give_up = 0;                         // self-test: the grid barrier whose waits run out, or 0
     float2 *tw1 = nullptr, *tw2 = nullptr;   // exp(-2 pi i m / n1), exp(-2 pi i m / n2), one buffer
     CUtensorMap tmap;  // 64-byte aligned by its own declaration
     CUtensorMap tmap_spread;  // box of one strip patch of the FP32 tiled spread

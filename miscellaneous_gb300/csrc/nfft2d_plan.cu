@@ -852,6 +852,7 @@ struct OneBinArgs {
     int chunk;
     int *status;
     int *host;  // page-locked copy of status[0], status[1], or null
+    int give_up;  // grid_wait's
 };
 
 template <typename CT, typename RecT>
@@ -886,7 +887,10 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
         r[u].mu = (mu1 << 16) | mu2;
         r[u].orig = i;
     }
-    if (!grid_wait(a.status, kGridCtas)) return;  // the counters are zero
+    if (!grid_wait(a.status, 1, a.give_up)) {  // the counters are zero
+        grid_done(a.status, true);
+        return;
+    }
     if (bad) latch_error(a.status, kErrNonfinite);
 #pragma unroll
     for (int u = 0; u < kOneBinItems; ++u) {
@@ -896,7 +900,10 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
         const unsigned t = have ? key[u] / cpt : 0xffffffffu, same = __match_any_sync(0xffffffffu, t);
         if (have && lane == __ffs(same) - 1) atomicAdd(a.tile_count + t, static_cast<unsigned>(__popc(same)));
     }
-    if (!grid_barrier(a.status, 2 * kGridCtas)) return;
+    if (!grid_barrier(a.status, 2, a.give_up)) {
+        grid_done(a.status, true);
+        return;
+    }
     // where every tile's points and work items start, in each CTA: (points,
     // items) scanned as one 64-bit word
     unsigned long long before = 0;
@@ -955,7 +962,10 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
                 make_int4(t, static_cast<int>(tile_start[t] + c * a.chunk),
                           static_cast<int>(min(count - c * a.chunk, static_cast<unsigned>(a.chunk))), 0);
     }
-    if (!grid_barrier(a.status, 3 * kGridCtas)) return;
+    if (!grid_barrier(a.status, 3, a.give_up)) {
+        grid_done(a.status, true);
+        return;
+    }
 #pragma unroll
     for (int u = 0; u < kOneBinItems; ++u) {
         const int i = gid + u * kStride;
@@ -964,7 +974,7 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
         static_cast<RecT *>(a.recs)[q] = r[u];
         a.src[q] = i;
     }
-    grid_done(a.status);
+    grid_done(a.status, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -2165,6 +2175,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
         a.chunks = p->chunks, a.chunk = p->chunk;
         a.status = p->d_status;
         a.host = async ? nullptr : p->h_status;
+        a.give_up = p->give_up;
         if (!async) p->h_status[0] = -1;  // until the kernel has the counts
         NFFT_TRY_CUDA(launch_one_bin(p, coord_dtype, a));
         if (coords_read) NFFT_TRY_CUDA(cudaEventRecord(coords_read, p->stream));
@@ -2246,10 +2257,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
     // the read-back is one small DMA, or the kernel's own write
     if (!one) NFFT_TRY_CUDA(cudaMemcpyAsync(p->h_status, p->d_status, 4 * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     NFFT_TRY_CUDA(cudaStreamSynchronize(p->stream));
-    if (one && hs[0] < 0) {  // given up on at a barrier
-        NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status + kBarrierWord, 0, 2 * sizeof(int), p->stream));
-        return NFFT2D_ERR_DEVICE_TIMEOUT;
-    }
+    if (one && hs[0] < 0) return NFFT2D_ERR_DEVICE_TIMEOUT;  // given up on at a barrier
     if (hs[1] & kErrNonfinite) return NFFT2D_ERR_NONFINITE;
     if (hs[1] & kErrTimeout) return NFFT2D_ERR_DEVICE_TIMEOUT;
     if (hs[0] < 0 || hs[0] > p->chunks_cap) return NFFT2D_ERR_INTERNAL;
@@ -2502,10 +2510,7 @@ int nfft2d::apply_status(nfft2d_plan_s *p) {
     // they are read (the stream is idle here)
     const int bits = hs[1];
     if (bits) NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status + 1, 0, sizeof(int), p->stream));
-    if (bits & kErrTimeout) {  // a grid barrier that was given up on leaves its words behind
-        NFFT_TRY_CUDA(cudaMemsetAsync(p->d_status + kBarrierWord, 0, 2 * sizeof(int), p->stream));
-        return NFFT2D_ERR_DEVICE_TIMEOUT;
-    }
+    if (bits & kErrTimeout) return NFFT2D_ERR_DEVICE_TIMEOUT;
     if (bits & kErrBounds) return NFFT2D_ERR_DEVICE_BOUNDS;
     return NFFT2D_OK;
 }
@@ -2525,6 +2530,12 @@ int nfft2d_plan_selftest_wait_timeout(nfft2d_plan p, int spin_limit) {
     if (!p || spin_limit < 1) return NFFT2D_ERR_INVALID_ARG;
     nfft2d::k_selftest_latch<<<1, 32, 0, p->stream>>>(static_cast<uint32_t>(spin_limit), p->d_status);
     NFFT_TRY_CUDA(cudaGetLastError());
+    return NFFT2D_OK;
+}
+
+int nfft2d_plan_selftest_barrier(nfft2d_plan p, int barrier) {
+    if (!p || barrier < 0 || barrier > 3) return NFFT2D_ERR_INVALID_ARG;
+    p->give_up = barrier;
     return NFFT2D_OK;
 }
 

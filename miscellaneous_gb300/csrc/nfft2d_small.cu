@@ -41,7 +41,8 @@ constexpr int kSmallSide = 512;    // longest FFT
 
 struct SmallArgs {
     int N1, N2, logn1, logn2;
-    float s;  // exponent sign
+    float s;      // exponent sign
+    int give_up;  // grid_wait's
     const float *d1, *d2;
     const float2 *tw1, *tw2;  // exp(-2 pi i m / n)
 };
@@ -186,7 +187,10 @@ __global__ void __launch_bounds__(kSmallThreads)
         for (int r = lane; r < n1; r += 32) inner[static_cast<size_t>(r) * g.C + c] = x[r];
         __syncwarp();
     }
-    if (!grid_barrier(ka.status, kSmallCtas)) return;
+    if (!grid_barrier(ka.status, 1, a.give_up)) {
+        grid_done(ka.status, true);
+        return;
+    }
     for (int r = gw; r < n1; r += kSmallWarps) {  // rows, with their halo images
         float2 *row = inner + static_cast<size_t>(r) * g.C;
 #pragma unroll 4
@@ -232,7 +236,10 @@ __global__ void __launch_bounds__(kSmallThreads)
         weights_poly2<K>(__int_as_float(raw.x), __int_as_float(raw.y), w1, w2, ka.poly);
 #pragma unroll
         for (int k = 0; k < S::W; ++k) w1s[k * S::WROW] = w1[k];
-        if (waiting && !grid_wait(ka.status, 2 * kSmallCtas)) return;
+        if (waiting && !grid_wait(ka.status, 2, a.give_up)) {
+            grid_done(ka.status, true);
+            return;
+        }
         waiting = false;
         if (p < B && q.count > 0) {  // a new tile
             const float2 *src = grid + static_cast<size_t>(q.r0 - K + H) * g.C + (q.c0 - S::KE + H);
@@ -294,7 +301,7 @@ __global__ void __launch_bounds__(kSmallThreads)
             q = small_unit<B>(chunks, u, units, split, g);
         }
     } while (u < units);
-    grid_done(ka.status);
+    grid_done(ka.status, false);
 }
 
 template <int K>
@@ -377,7 +384,10 @@ __global__ void __launch_bounds__(kSmallThreads)
         }
         fence_proxy_async_smem();  // the patch, before the TMA engine reads it
         // the zeros of the grid are there (and so is the loop's code) by now
-        if (waiting && !grid_wait(ka.status, kSmallCtas)) return;
+        if (waiting && !grid_wait(ka.status, 1, a.give_up)) {
+            grid_done(ka.status, true);
+            return;
+        }
         waiting = false;
         __syncwarp();
         pending = true;
@@ -389,7 +399,10 @@ __global__ void __launch_bounds__(kSmallThreads)
     }
     if (lane == 0) bulk_wait_all();
     __syncwarp();
-    if (!grid_barrier(ka.status, 2 * kSmallCtas)) return;
+    if (!grid_barrier(ka.status, 2, a.give_up)) {
+        grid_done(ka.status, true);
+        return;
+    }
     for (int r = gw; r < n1; r += kSmallWarps) {  // rows with their halo images folded in
         float2 *row = inner + static_cast<size_t>(r) * g.C;
         const bool edge = r < H || r >= n1 - H;
@@ -415,7 +428,10 @@ __global__ void __launch_bounds__(kSmallThreads)
         }
         __syncwarp();
     }
-    if (!grid_barrier(ka.status, 3 * kSmallCtas)) return;
+    if (!grid_barrier(ka.status, 3, a.give_up)) {
+        grid_done(ka.status, true);
+        return;
+    }
     for (int bc = gw; bc < N2; bc += kSmallWarps) {  // band columns, cropped
         const int j = bc < N2 / 2 ? bc + N2 / 2 : bc - N2 / 2, c = bc < N2 / 2 ? bc : n2 - N2 + bc;
         const float s2 = __ldg(a.d2 + j);
@@ -431,7 +447,7 @@ __global__ void __launch_bounds__(kSmallThreads)
         }
         __syncwarp();
     }
-    grid_done(ka.status);
+    grid_done(ka.status, false);
 }
 
 SmallArgs small_args(const nfft2d_plan_s *p, int sign) {
@@ -441,6 +457,7 @@ SmallArgs small_args(const nfft2d_plan_s *p, int sign) {
     while ((1 << a.logn1) < p->g.n1) ++a.logn1;
     while ((1 << a.logn2) < p->g.n2) ++a.logn2;
     a.s = sign < 0 ? -1.f : 1.f;
+    a.give_up = p->give_up;
     a.d1 = static_cast<const float *>(p->deap1);
     a.d2 = static_cast<const float *>(p->deap2);
     a.tw1 = p->tw1;
