@@ -255,8 +255,9 @@ int nfft2d_selftest_wait_timeout(int spin_limit, void *stream);
 int nfft2d_plan_selftest_wait_timeout(nfft2d_plan plan, int spin_limit);
 /* The plan's one-launch binning and transforms give up at their grid barrier
  * `barrier` (1 to 3) from the next call on, as they do when a wait runs out;
- * 0 ends that.  The next nfft2d_synchronize reports
- * NFFT2D_ERR_DEVICE_TIMEOUT.  Host only. */
+ * 0 ends that.  A set_points reports NFFT2D_ERR_DEVICE_TIMEOUT (an
+ * asynchronous one at the next nfft2d_synchronize) and leaves no points, a
+ * transform at the next nfft2d_synchronize.  Host only. */
 int nfft2d_plan_selftest_barrier(nfft2d_plan plan, int barrier);
 
 /* ---- exact direct sum ----------------------------------------------------

@@ -19,6 +19,7 @@ constexpr int kMaxK = 8;
 constexpr int kErrTimeout = 1;
 constexpr int kErrBounds = 2;
 constexpr int kErrNonfinite = 4;
+constexpr int kErrBinning = 8;  // with kErrTimeout: the wait that ran out was the binning's
 
 // d_status: [0] work items, [1] error bits, [2] the spread's work counter, [3]
 // its own work items, [4] [5] the grid barrier of the one-launch transforms

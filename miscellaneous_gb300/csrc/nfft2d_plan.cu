@@ -851,9 +851,27 @@ struct OneBinArgs {
     int4 *chunks;
     int chunk;
     int *status;
-    int *host;  // page-locked copy of status[0], status[1], or null
+    int *host;  // page-locked: status[0], status[1], and [2] not 0 if a wait has run out; or null
     int give_up;  // grid_wait's
 };
+
+// The end of k_bin_one on every way out.  If a wait has run out, one thread
+// tells the host and leaves points that any transform may read: all in cell 0
+// and in no work item.
+template <typename RecT>
+__device__ __forceinline__ void bin_one_done(const OneBinArgs &a, bool complete) {
+    if (!complete && threadIdx.x == 0) latch_error(a.status, kErrBinning);
+    if (!grid_done(a.status, !complete)) return;
+    __threadfence();
+    for (int i = 0; i < a.M; ++i) {
+        RecT r{};
+        r.orig = i;
+        static_cast<RecT *>(a.recs)[i] = r;
+        a.src[i] = i;
+    }
+    atomicExch(a.status, 0);
+    if (a.host) a.host[2] = 1;
+}
 
 template <typename CT, typename RecT>
 __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_constant__ OneBinArgs a) {
@@ -887,10 +905,7 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
         r[u].mu = (mu1 << 16) | mu2;
         r[u].orig = i;
     }
-    if (!grid_wait(a.status, 1, a.give_up)) {  // the counters are zero
-        grid_done(a.status, true);
-        return;
-    }
+    if (!grid_wait(a.status, 1, a.give_up)) return bin_one_done<RecT>(a, false);  // the counters are zero
     if (bad) latch_error(a.status, kErrNonfinite);
 #pragma unroll
     for (int u = 0; u < kOneBinItems; ++u) {
@@ -900,10 +915,7 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
         const unsigned t = have ? key[u] / cpt : 0xffffffffu, same = __match_any_sync(0xffffffffu, t);
         if (have && lane == __ffs(same) - 1) atomicAdd(a.tile_count + t, static_cast<unsigned>(__popc(same)));
     }
-    if (!grid_barrier(a.status, 2, a.give_up)) {
-        grid_done(a.status, true);
-        return;
-    }
+    if (!grid_barrier(a.status, 2, a.give_up)) return bin_one_done<RecT>(a, false);
     // where every tile's points and work items start, in each CTA: (points,
     // items) scanned as one 64-bit word
     unsigned long long before = 0;
@@ -962,19 +974,17 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
                 make_int4(t, static_cast<int>(tile_start[t] + c * a.chunk),
                           static_cast<int>(min(count - c * a.chunk, static_cast<unsigned>(a.chunk))), 0);
     }
-    if (!grid_barrier(a.status, 3, a.give_up)) {
-        grid_done(a.status, true);
-        return;
-    }
+    if (!grid_barrier(a.status, 3, a.give_up)) return bin_one_done<RecT>(a, false);
 #pragma unroll
     for (int u = 0; u < kOneBinItems; ++u) {
         const int i = gid + u * kStride;
         if (i >= a.M) continue;
         const unsigned q = __ldcg(a.cell_count + key[u]) + rank[u];
+        if (q >= static_cast<unsigned>(a.M)) continue;  // never, unless the counters are not this launch's
         static_cast<RecT *>(a.recs)[q] = r[u];
         a.src[q] = i;
     }
-    grid_done(a.status, false);
+    bin_one_done<RecT>(a, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -2176,7 +2186,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
         a.status = p->d_status;
         a.host = async ? nullptr : p->h_status;
         a.give_up = p->give_up;
-        if (!async) p->h_status[0] = -1;  // until the kernel has the counts
+        if (!async) p->h_status[0] = -1, p->h_status[2] = 0;  // until the kernel has the counts
         NFFT_TRY_CUDA(launch_one_bin(p, coord_dtype, a));
         if (coords_read) NFFT_TRY_CUDA(cudaEventRecord(coords_read, p->stream));
     } else {
@@ -2257,7 +2267,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
     // the read-back is one small DMA, or the kernel's own write
     if (!one) NFFT_TRY_CUDA(cudaMemcpyAsync(p->h_status, p->d_status, 4 * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     NFFT_TRY_CUDA(cudaStreamSynchronize(p->stream));
-    if (one && hs[0] < 0) return NFFT2D_ERR_DEVICE_TIMEOUT;  // given up on at a barrier
+    if (one && (hs[0] < 0 || hs[2])) return NFFT2D_ERR_DEVICE_TIMEOUT;
     if (hs[1] & kErrNonfinite) return NFFT2D_ERR_NONFINITE;
     if (hs[1] & kErrTimeout) return NFFT2D_ERR_DEVICE_TIMEOUT;
     if (hs[0] < 0 || hs[0] > p->chunks_cap) return NFFT2D_ERR_INTERNAL;
@@ -2505,6 +2515,11 @@ int nfft2d::apply_status(nfft2d_plan_s *p) {
         }
         if (hs[0] < 0 || hs[0] > p->chunks_cap) return NFFT2D_ERR_INTERNAL;
         p->n_chunks = hs[0];
+        if (hs[1] & kErrBinning) {  // unsorted points: none
+            p->points_valid = false;
+            p->M = 0;
+            p->n_chunks = 0;
+        }
     }
     // a device-side error is reported once: the bits are cleared after
     // they are read (the stream is idle here)

@@ -1,6 +1,7 @@
-"""A grid barrier of the one-launch transforms that is given up on (by a plan's own
-self-test switch: no wait, no stalled GPU) is reported and leaves the barrier
-ready for the next launch, whatever the host calls in between.
+"""A grid barrier of the one-launch binning or transforms that is given up on
+(by a plan's own self-test switch: no wait, no stalled GPU) is reported, leaves
+points that later calls read in bounds, and leaves the barrier ready for the
+next launch, whatever the host calls in between.
 
 Tolerance: the spread adds in any order, 1e-6 relative in FP32; the forward
 sums in a fixed one."""
@@ -17,7 +18,8 @@ def _data(precision):
     g.manual_seed(8)
     c = torch.complex64 if precision == "f32" else torch.complex128
     x = [torch.rand(M, generator=g, device="cuda") - 0.5 for _ in range(2)]
-    return x, torch.randn(N, N, generator=g, device="cuda", dtype=c), torch.randn(M, generator=g, device="cuda", dtype=c)
+    far = [torch.rand(3 * M, generator=g, device="cuda") - 0.5 for _ in range(2)]
+    return x, far, torch.randn(N, N, generator=g, device="cuda", dtype=c), torch.randn(M, generator=g, device="cuda", dtype=c)
 
 
 def _reference(precision, x, F, f):
@@ -49,10 +51,39 @@ def _expect(status, call):
     assert e.value.status == getattr(_lib, status)
 
 
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("barrier", [1, 2, 3])
+def test_binning(barrier, precision):
+    from miscellaneous_gb300.nfft import Plan
+    x, far, F, f = _data(precision)
+    want = _reference(precision, x, F, f)
+    with Plan(N, N, precision=precision) as p:
+        p.set_points(*far)  # records of points that the next set does not have
+        for _ in range(2):
+            _give_up(p, barrier)
+            _expect("ERR_DEVICE_TIMEOUT", lambda: p.set_points(*x))
+            _expect("ERR_NO_POINTS", lambda: p.forward(F))
+            _give_up(p, 0)
+            _good(p, x, F, f, want)  # straight after: the barrier's words are zero
+        for direct in (False, True):  # every gather and spread reads those points in bounds
+            p.set_points(*far)
+            _give_up(p, barrier)
+            p.set_points(*x, sync=False)
+            _give_up(p, 0)
+            if precision == "f32":
+                p.set_tuning(gather_variant=2 if direct else 1, spread_variant=2 if direct else 1)
+            p.forward(F), p.adjoint(f)
+            _expect("ERR_DEVICE_TIMEOUT", p.synchronize)
+            _expect("ERR_NO_POINTS", lambda: p.forward(F))
+            p.synchronize()  # reported once
+            p.set_tuning(gather_variant=0, spread_variant=0)
+            _good(p, x, F, f, want, sync=False)
+
+
 @pytest.mark.parametrize("adjoint,barrier", [(False, 1), (False, 2), (True, 1), (True, 2), (True, 3)])
 def test_transforms(adjoint, barrier):
     from miscellaneous_gb300.nfft import Plan
-    x, F, f = _data("f32")
+    x, _, F, f = _data("f32")
     want = _reference("f32", x, F, f)
     with Plan(N, N) as p:
         p.set_points(*x)
