@@ -489,13 +489,6 @@ FftArgs fft_args(const nfft2d_plan_s *p, int sign) {
     return a;
 }
 
-// Dynamic shared memory above the 48 KB default needs an opt-in per kernel.
-template <typename KernelT>
-cudaError_t allow_smem(KernelT kernel, int smem) {
-    if (smem > 48 * 1024) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return cudaSuccess;
-}
-
 }  // namespace
 
 bool fused_fft_eligible(int precision, int n1, int n2) {

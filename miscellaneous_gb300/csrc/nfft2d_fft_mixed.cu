@@ -460,10 +460,8 @@ int block_threads(const Geom &g, int elems) {
 template <typename Kernel, typename... Args>
 cudaError_t launch(Kernel kernel, const nfft2d_plan_s *p, bool after, int blocks, int elems, Args... args) {
     const int smem = 2 * padded(elems) * static_cast<int>(sizeof(float2)) + 16;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
     if (after) return launch_after(kernel, dim3(blocks), block_threads(p->g, elems), smem, p->stream, args...);
     kernel<<<blocks, block_threads(p->g, elems), smem, p->stream>>>(args...);
     return cudaGetLastError();

@@ -344,10 +344,10 @@ __global__ void __launch_bounds__(kThreads, K <= 6 ? 3 : 2)
     g2[io] = a.ds2 * (v.x * bx + v.y * by);
 }
 
+// Two patches of the largest tile (64 x 64, K = 8) are 103 KB.
 template <typename KernelT>
 cudaError_t prepare_smem(KernelT kernel, int smem) {
-    if (smem > 48 * 1024) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return cudaSuccess;
+    return allow_smem(kernel, smem, 128 * 1024);
 }
 
 template <int K, int MODE>

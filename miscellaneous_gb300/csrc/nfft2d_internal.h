@@ -342,6 +342,17 @@ cudaError_t launch_after(Kernel kernel, dim3 grid, int threads, int smem, cudaSt
     return launch_chained(true, kernel, grid, threads, smem, stream, args...);
 }
 
+// Dynamic shared memory above the 48 KB default needs a limit per kernel, which
+// the whole process shares: always `most`, never this launch's need, or a thread
+// would lower what another's launch is about to use.  Most a CTA can have: 227
+// KB, its static shared memory included.
+constexpr int kMaxSmem = 227 * 1024;
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, int smem, int most = kMaxSmem) {
+    if (smem <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // The fused FFT passes (nfft2d_fft.cu): eligibility, per-plan twiddle tables,
 // type 2 = deapodize/pad + band-column FFT, then row FFT + halo fill;
 // type 1 = halo fold + row FFT, then band-column FFT + crop/deapodize.

@@ -2038,7 +2038,8 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
         max_cells = std::max(max_cells, p->ncells);
     }
     const size_t smem = sizeof(unsigned) * (max_cells + 1 + 32);
-    if (smem > 200 * 1024) return NFFT2D_ERR_UNSUPPORTED;  // the counters must fit in shared memory
+    constexpr int kMost = 200 * 1024;
+    if (smem > kMost) return NFFT2D_ERR_UNSUPPORTED;  // the counters must fit in shared memory
     for (int i = 0; i < count; ++i) {
         nfft2d_plan_s *p = plans[i];
         const void *dx1 = x1[i], *dx2 = x2[i];
@@ -2086,7 +2087,7 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
     }
     NFFT_TRY_CUDA(cudaMemcpyAsync(space.d_jobs, space.h_jobs, sizeof(SmallBinJob) * count, cudaMemcpyHostToDevice, stream));
     auto kernel = coord_dtype == NFFT2D_COORD_F64 ? k_bin_small<double> : k_bin_small<float>;
-    NFFT_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    NFFT_TRY_CUDA(allow_smem(kernel, static_cast<int>(smem), kMost));
     kernel<<<count, kSmallBinThreads, smem, stream>>>(space.d_jobs);
     NFFT_TRY_CUDA(cudaGetLastError());
     NFFT_TRY_CUDA(cudaStreamSynchronize(stream));

@@ -807,9 +807,9 @@ extern "C" int nfft2d_nufft3_2d(const double *x, const double *y, const double *
     const size_t rb = dbl ? sizeof(double) : sizeof(float);
     const T3Shape shape = t3_shape(W);
     int B = 32;  // points per weight batch of the FP64 spread
-    while (dbl && B > 4 && t3_spread_smem(W, B) > 227 * 1024) B /= 2;
+    while (dbl && B > 4 && t3_spread_smem(W, B) > nfft2d::kMaxSmem) B /= 2;
     const size_t smem = dbl ? t3_spread_smem(W, B) : shape.spread_smem;
-    if (smem > 227 * 1024 || shape.gather_smem > 227 * 1024) return NFFT2D_ERR_UNSUPPORTED;
+    if (smem > nfft2d::kMaxSmem || shape.gather_smem > nfft2d::kMaxSmem) return NFFT2D_ERR_UNSUPPORTED;
     const size_t cells = static_cast<size_t>(P.Mrx) * P.Mry;
     const size_t csz = 2 * rb;
     const int tiles_x = (P.Mrx + kT3Tile - 1) / kT3Tile, tiles_y = (P.Mry + kT3Tile - 1) / kT3Tile;
@@ -890,7 +890,7 @@ extern "C" int nfft2d_nufft3_2d(const double *x, const double *y, const double *
                                                      words(bi.counts));
         T3_CUDA(cudaGetLastError());
         T3_CUDA(bin(tmp, bi, len_in, item_in));
-        T3_CUDA(cudaFuncSetAttribute(k_t3_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        T3_CUDA(nfft2d::allow_smem(k_t3_spread, static_cast<int>(smem)));
         k_t3_spread<<<static_cast<unsigned>(max_items), kT3Warps * 32, smem, st>>>(
             reinterpret_cast<const T3Rec *>(base + bi.recs), items, words(bi.counts) + ntiles, P, tiles_x, B,
             static_cast<double *>(S.grid));
@@ -905,7 +905,7 @@ extern "C" int nfft2d_nufft3_2d(const double *x, const double *y, const double *
         T3_CUDA(cudaGetLastError());
         T3_CUDA(bin(tmp, bi, len_in, item_in));
         auto spread = shape.spread_threads <= 128 ? k_t3_spread_f32<128, 4> : k_t3_spread_f32<448, 1>;
-        T3_CUDA(cudaFuncSetAttribute(spread, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        T3_CUDA(nfft2d::allow_smem(spread, static_cast<int>(smem)));
         spread<<<static_cast<unsigned>(max_items), shape.spread_threads, smem, st>>>(
             reinterpret_cast<const T3Rec32 *>(base + bi.recs), items, words(bi.counts) + ntiles, P, tiles_x, shape.PR,
             shape.PC, prex, tabo_x, prey, tabo_y, reinterpret_cast<float2 *>(base + off_grid));
@@ -931,7 +931,7 @@ extern "C" int nfft2d_nufft3_2d(const double *x, const double *y, const double *
         T3Freq *tmp = reinterpret_cast<T3Freq *>(base + bo.tmp);
         double2 *factor = reinterpret_cast<double2 *>(base + off_factor);
         auto gather = shape.gather_threads <= 128 ? k_t3_gather_f32<128, 4> : k_t3_gather_f32<448, 1>;
-        T3_CUDA(cudaFuncSetAttribute(gather, cudaFuncAttributeMaxDynamicSharedMemorySize, shape.gather_smem));
+        T3_CUDA(nfft2d::allow_smem(gather, shape.gather_smem));
         for (long long at = 0; at < len_out; at += slice) {
             const long long n = std::min(slice, len_out - at);
             if (at > 0) T3_CUDA(cudaMemsetAsync(words(bo.counts), 0, static_cast<size_t>(ntiles + 1) * sizeof(unsigned), st));
