@@ -135,12 +135,26 @@ typedef struct {
                               order).  Set it before set_points or after. */
 } nfft2d_tuning;
 
+/* Which kernels a plan's calls run at present, for its points and tuning (the
+ * same work with the same results; sizes decide). */
+typedef struct {
+    int binning;           /* of the points set last: 0 no points, 1 separate
+                              passes, 2 one launch                              */
+    int forward, adjoint;  /* type 2, type 1: 0 a kernel a stage, 1 one launch
+                              (small transforms; not while timing is enabled)   */
+    int gather;            /* of a forward in stages, and of bin_and_forward's:
+                              0 tiled, 1 direct, 2 on the tensor cores          */
+} nfft2d_paths;
+
 #define NFFT2D_ORDER_CALLER 0
 #define NFFT2D_ORDER_BINNED 1
 
 /* Stage times in milliseconds, from CUDA events recorded on the plan's
- * stream while timing is enabled.  Each field holds the most recent run of
- * that stage: a type-2 call refreshes pad / fft_type2 / halo_fill / gather,
+ * stream while timing is enabled.  Every stage is then a kernel of its own
+ * that starts when the one before has ended, so the stages add up to more than
+ * a call without timing takes, and small transforms, which otherwise run in
+ * one launch (nfft2d_paths), to about twice that: time whole calls to compare
+ * settings.  Each field holds the most recent run of that stage: a type-2 call refreshes pad / fft_type2 / halo_fill / gather,
  * a type-1 call refreshes spread / fold / fft_type1 / crop, set_points
  * refreshes sort; fields of stages that never ran are 0. */
 typedef struct {
@@ -167,6 +181,7 @@ int nfft2d_plan_destroy(nfft2d_plan plan);
 int nfft2d_set_stream(nfft2d_plan plan, void *stream);
 int nfft2d_set_tuning(nfft2d_plan plan, const nfft2d_tuning *tuning);
 int nfft2d_get_info(nfft2d_plan plan, nfft2d_info *info);
+int nfft2d_get_paths(nfft2d_plan plan, nfft2d_paths *paths);
 
 /* The binned order of the points set last: perm[i] = the caller's index of
  * the point at binned position i (M ints, DEVICE).  Asynchronous on the

@@ -52,6 +52,13 @@ class Info(ctypes.Structure):
         return {name: getattr(self, name) for name, _ in self._fields_}
 
 
+class Paths(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int) for n in ("binning", "forward", "adjoint", "gather")]
+
+    def as_dict(self) -> dict:
+        return {name: getattr(self, name) for name, _ in self._fields_}
+
+
 ORDER_CALLER = 0
 ORDER_BINNED = 1
 
@@ -115,6 +122,7 @@ _SIGNATURES = {
     "nfft2d_set_stream": (_I, [_P, _P]),
     "nfft2d_set_tuning": (_I, [_P, ctypes.POINTER(Tuning)]),
     "nfft2d_get_info": (_I, [_P, ctypes.POINTER(Info)]),
+    "nfft2d_get_paths": (_I, [_P, ctypes.POINTER(Paths)]),
     "nfft2d_get_permutation": (_I, [_P, _P]),
     "nfft2d_layout_query": (_I, [_I, _I, _D, _I, _I, _I, ctypes.POINTER(Info)]),
     "nfft2d_set_points": (_I, [_P, _LL, _P, _P, _I, _I]),

@@ -378,7 +378,7 @@ cudaError_t launch_K(const nfft2d_plan_s *p, void *f, const void *v, void *g1, v
             static_cast<const double2 *>(v), static_cast<double *>(g1), static_cast<double *>(g2), a, p->poly64);
     } else if constexpr (MODE == 0) {
         if constexpr (K >= 6) {
-            if (tc_gather_pays(K, p->g, p->M)) {
+            if (tc_gather(p)) {
                 const long long items = p->n_chunks >= 0 ? p->n_chunks : p->chunks_cap;
                 auto kernel = p->compensated ? k_gather_tc<K, true> : k_gather_tc<K, false>;
                 const cudaError_t e = prepare_smem(kernel, TcGeo<K>::SMEM);
@@ -424,6 +424,10 @@ cudaError_t launch_gather(const nfft2d_plan_s *p, void *f, bool after) {
 
 cudaError_t launch_grad(const nfft2d_plan_s *p, const void *v, void *g1, void *g2) {
     return dispatch<1>(p, nullptr, v, g1, g2, true);
+}
+
+bool tc_gather(const nfft2d_plan_s *p) {
+    return p->precision == NFFT2D_F32 && p->gather_variant != NFFT2D_VARIANT_TILED && tc_gather_pays(p->K, p->g, p->M);
 }
 
 int gather_smem_bytes(const nfft2d_plan_s *p) { return 2 * patch_stride_elems(p->g) * static_cast<int>(sizeof(float2)) + 128; }

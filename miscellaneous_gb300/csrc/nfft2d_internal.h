@@ -125,6 +125,7 @@ struct nfft2d_plan_s {
     nfft2d::WinPoly poly{};      // FP32 window polynomials
     nfft2d::WinPoly64 poly64{};  // FP64 window polynomials (FP64 plans)
     int chunk = 256;
+    int binning = 0;  // nfft2d_paths
     int gather_variant = NFFT2D_VARIANT_TILED;
     bool gather_auto = true;     // FP32: pick the gather by bin density at set_points
     int spread_variant = NFFT2D_VARIANT_TILED;
@@ -204,6 +205,7 @@ cudaError_t launch_halo_fold(const nfft2d_plan_s *p);
 cudaError_t launch_gather(const nfft2d_plan_s *p, void *f, bool after = true);
 cudaError_t launch_grad(const nfft2d_plan_s *p, const void *v, void *g1, void *g2);
 int gather_smem_bytes(const nfft2d_plan_s *p);
+bool tc_gather(const nfft2d_plan_s *p);  // the forward's gather runs on the tensor cores
 
 // spread.cu
 cudaError_t launch_spread(const nfft2d_plan_s *p, const void *f);

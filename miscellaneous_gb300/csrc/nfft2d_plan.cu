@@ -1977,6 +1977,16 @@ int nfft2d_get_info(nfft2d_plan p, nfft2d_info *info) {
     return NFFT2D_OK;
 }
 
+int nfft2d_get_paths(nfft2d_plan p, nfft2d_paths *paths) {
+    if (!p || !paths) return NFFT2D_ERR_INVALID_ARG;
+    const bool points = p->points_valid && p->M > 0;
+    paths->binning = points ? p->binning : 0;
+    paths->forward = points && use_small(p, false);
+    paths->adjoint = points && use_small(p, true);
+    paths->gather = p->gather_variant == NFFT2D_VARIANT_TILED ? 0 : (points && tc_gather(p) ? 2 : 1);
+    return NFFT2D_OK;
+}
+
 static int nfft2d_set_points_impl(nfft2d_plan p, long long M, const void *x1, const void *x2, int coord_dtype, int units,
                                   bool async) {
     if (!p) return NFFT2D_ERR_INVALID_ARG;
@@ -2177,6 +2187,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
     stage_begin(p, ST_SORT);
     const int *hs = p->h_status;  // page-locked
     const bool one = use_one_bin(p, M, coords_read != nullptr);
+    p->binning = one ? 2 : 1;
     if (one) {
         OneBinArgs a{};
         a.x1 = x1, a.x2 = x2, a.M = static_cast<int>(M);

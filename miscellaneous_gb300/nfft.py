@@ -147,6 +147,12 @@ class Plan:
         check(self._lib.nfft2d_get_info(self._h, ctypes.byref(i)), "nfft2d_get_info")
         return i.as_dict()
 
+    def paths(self) -> dict:
+        """The kernels the plan's calls run at present (nfft2d_paths)."""
+        t = _lib.Paths()
+        check(self._lib.nfft2d_get_paths(self._h, ctypes.byref(t)), "nfft2d_get_paths")
+        return t.as_dict()
+
     def enable_timing(self, on: bool = True) -> None:
         check(self._lib.nfft2d_enable_timing(self._h, int(bool(on))), "nfft2d_enable_timing")
 
