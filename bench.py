@@ -828,9 +828,11 @@ def run_ours(args, wl):
         sharded.adjoint(f, out=F_out)  # this rank's points, then the sum all-reduce (N > 1)
 
     # the timed steps run without the plan's per-stage events (recording them
-    # costs ~10 % of a polar step); the stage breakdown comes from as many
-    # further steps with them, after the timed region
+    # costs ~10 % of a polar step, and keeps the stages apart); the stage
+    # breakdown comes from as many further steps with them, after the timed
+    # region
     plan.enable_timing(False)
+    paths = plan.paths()
     for _ in range(args.warmup):
         step()
         flush.zero_()
@@ -1142,11 +1144,13 @@ def run_ours(args, wl):
             "precision_study": study,
             "binned_io": binned,
             "spread_small_cases": small,
-            "gpu_launches": 7 * args.steps,
-            "gpu_launches_note": ("our kernels in the timed region per step: column FFT+pad, row FFT+fill, gather, "
-                                  "grid zeroing, spread, fold+row FFT, column FFT+crop") if fused else
-                                 ("our kernels in the timed region per step: pad, halo_fill, gather, grid zeroing, "
-                                  "spread, fold, crop (cuFFT kernels not counted)"),
+            "gpu_launches": ((1 if paths["forward"] else 3) + (1 if paths["adjoint"] else 4)) * args.steps,
+            "gpu_launches_note": "our kernels in the timed region per step: " + ", ".join((
+                ["the forward in one launch"] if paths["forward"] else
+                ["column FFT+pad", "row FFT+fill", "gather"] if fused else ["pad", "halo_fill", "gather"]) + (
+                ["the adjoint in one launch"] if paths["adjoint"] else
+                ["grid zeroing", "spread", "fold+row FFT", "column FFT+crop"] if fused else
+                ["grid zeroing", "spread", "fold", "crop (cuFFT kernels not counted)"])),
             "clocks": clocks.summary(),
         }
         print(json.dumps(line))
