@@ -9,10 +9,23 @@
 // column weights in shared memory as a row of the A operand, and finishes its
 // own accumulator lane with the row weights.
 //
-// Precision: every operand is the sum of three bf16 parts (8 + 8 + 8
-// significant bits), the six products down to 2^-18 are taken, and the leading
-// one has an accumulator of its own in which nothing is rounded (see
-// split_weight).  bf16 keeps FP32's exponent range: no scaling.
+// Precision: every operand is a sum of three bf16 parts, and the six largest of
+// the nine products are taken, the leading one in an accumulator of its own.
+// bf16 keeps FP32's exponent range: no scaling.  What is left out:
+//   - values: nothing down to 2^-27 of the value.
+//   - weights: 2^-27 of the window's peak, or 2^-18 of a weight below 2^-9 of it,
+//     whose leading part is zero (see split_weight).
+//   - the three smallest products: 2^-26 of peak times value, or 2^-17 of weight
+//     times value for those weights.
+//   - the unit's sums, truncated at about 2^-24 of the largest term: nothing of
+//     the leading products while the cells under a window differ by less than 2^6
+//     or so, up to that unit a product where they differ by more.
+// Relative error against 64 bits, the FP32 gather -> here (512^2 coefficients,
+// 2^20 points, w 6 | 7 | 8): random coefficients 2.41 -> 2.33e-7 | 2.71 -> 2.59 |
+// 3.31 -> 3.15; a regridder's raster 4.29 -> 4.30 (w 6); 100 scatterers under a
+// taper, whose peaks stand 2^30 above the cells around them, 1.58 -> 1.63 | 1.67 ->
+// 1.74 | 1.72 -> 1.77; at points where only the tails of their windows meet such
+// a peak the two agree to 2 digits, the FP32 window's own fit being larger.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -122,9 +135,10 @@ __device__ __forceinline__ Bf3 split_value(float x0, float x1) {
 }
 
 // Window weights, at most 1 in magnitude: h is a multiple of 2^-8 (rounded by
-// adding and taking back 1.5 * 2^15), so that its products with 8-bit parts,
-// summed over a window, fit the accumulator's 24 bits: the tensor cores
-// truncate, and a leading sum of rounded parts came out 0.9e-7 short.
+// adding and taking back 1.5 * 2^15), so that its products with 8-bit parts of
+// values of one size, summed over a window, fit the accumulator's 24 bits: the
+// tensor cores truncate, and with h rounded at each weight's own size a leading
+// sum came out 0.9e-7 short.
 __device__ __forceinline__ Bf3 split_weight(float x0, float x1) {
     constexpr float kMagic = 49152.f;
     const float2 x = make_float2(x0, x1);
