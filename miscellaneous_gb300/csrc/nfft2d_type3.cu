@@ -714,11 +714,11 @@ int cuda_status(cudaError_t e) {
 
 // Extents of both sets, {min, max} of x, y, s, t, with one read-back.
 int minmax(const double *x, const double *y, long long nx, const double *s, const double *t, long long ns,
-           unsigned long long *d_mm, cudaStream_t st, double out[8]) {
+           unsigned long long *d_mm, cudaStream_t st, int sms, double out[8]) {
     const unsigned long long init[8] = {~0ull, 0ull, ~0ull, 0ull, ~0ull, 0ull, ~0ull, 0ull};
     T3_CUDA(cudaMemcpyAsync(d_mm, init, sizeof init, cudaMemcpyHostToDevice, st));
     const long long n = std::max(nx, ns);
-    const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((n + 1023) / 1024, 152)));
+    const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((n + 1023) / 1024, sms)));
     k_minmax2<<<dim3(blocks, 2), kMinmaxThreads, 0, st>>>(x, y, nx, s, t, ns, d_mm);
     T3_CUDA(cudaGetLastError());
     unsigned long long h[8];
@@ -754,9 +754,12 @@ extern "C" int nfft2d_nufft3_2d(const double *x, const double *y, const double *
     if (len_in > (1LL << 40) || len_out > (1LL << 40)) return NFFT2D_ERR_INVALID_ARG;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     Scratch S{st};
+    int dev = 0, sms = 0;
+    T3_CUDA(cudaGetDevice(&dev));
+    T3_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     T3_CUDA(cudaMallocAsync(&S.mm, 8 * sizeof(unsigned long long), st));
     double ext[8];
-    const int rc = minmax(x, y, len_in, s, t, len_out, static_cast<unsigned long long *>(S.mm), st, ext);
+    const int rc = minmax(x, y, len_in, s, t, len_out, static_cast<unsigned long long *>(S.mm), st, sms, ext);
     if (rc != NFFT2D_OK) return rc;
     for (double v : ext)
         if (!std::isfinite(v)) return NFFT2D_ERR_NONFINITE;
@@ -814,11 +817,11 @@ extern "C" int nfft2d_nufft3_2d(const double *x, const double *y, const double *
     const size_t csz = 2 * rb;
     const int tiles_x = (P.Mrx + kT3Tile - 1) / kT3Tile, tiles_y = (P.Mry + kT3Tile - 1) / kT3Tile;
     const long long ntiles = static_cast<long long>(tiles_x) * tiles_y;
-    // FP32 work items: enough of them for each of the 152 SMs to hold several
-    // CTAs, a few batches each (a spread item ends in a patch of atomics, a
-    // gather item begins by reading one)
-    auto item_of = [](long long n) {
-        const long long v = n / (152 * 8) / 64 * 64;
+    // FP32 work items: enough of them for each SM to hold several CTAs, a few
+    // batches each (a spread item ends in a patch of atomics, a gather item
+    // begins by reading one)
+    auto item_of = [sms](long long n) {
+        const long long v = n / (sms * 8LL) / 64 * 64;
         return static_cast<unsigned>(std::max(128LL, std::min<long long>(v, 512)));
     };
     // FP32 frequencies go in slices, which bounds their work buffers
