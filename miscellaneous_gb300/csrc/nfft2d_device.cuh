@@ -270,13 +270,6 @@ __device__ __forceinline__ void weights_poly2(float t1, float t2, float (&w1)[2 
     weights_even<K, 2>(ts, ws, P);
 }
 
-template <int K>
-__device__ __forceinline__ void weights_poly1(float t, float (&w)[2 * K + 1], const WinPoly &P) {
-    const float ts[1] = {t};
-    float(*const ws[1])[2 * K + 1] = {&w};
-    weights_even<K, 1>(ts, ws, P);
-}
-
 // The taps and their derivatives d/dt from the same polynomials: Horner for
 // value and slope together (slope = slope * t + value before each value
 // step), two taps per packed FMA.  The slope of the fit differs from the

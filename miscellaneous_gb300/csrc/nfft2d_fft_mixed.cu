@@ -1,7 +1,8 @@
 // nfft2d_fft_mixed.cu -- the fused FFT passes (nfft2d_fft.cu) for sides that
-// are products of 2, 3, 5, 7, 11 and 13, with one larger prime: FP32 plans whose oversampled grid is
-// not a power of two a side, which otherwise run pad, a 2D library plan (two
-// kernels), halo fill -- fold, two, crop the other way.
+// are products of 2, 3, 5, 7, 11 and 13, with at most one larger prime: FP32
+// plans whose oversampled grid is not a power of two a side, which otherwise run
+// pad, a 2D library plan (two kernels), halo fill -- fold, two, crop the other
+// way.
 //
 // Same two passes a direction: P band columns a CTA with the pad or the crop,
 // a row a CTA with the halo's fill or fold.  One Stockham stage per factor (16
@@ -36,7 +37,7 @@ struct MixedFft {
 
 struct MixedArgs {
     MixedFft f;  // along the pass's direction
-    int N1, N2, n1, n2, H, C, Cl;
+    int N1, N2, n1, n2, H, C;
     int logP;
     float s;  // exponent sign
 };
@@ -437,7 +438,7 @@ MixedArgs mixed_args(const nfft2d_plan_s *p, int sign, int n) {
     MixedArgs a{};
     factor(n, &a.f);
     a.N1 = p->N1, a.N2 = p->N2, a.n1 = g.n1, a.n2 = g.n2;
-    a.H = g.H, a.C = g.C, a.Cl = g.Cl;
+    a.H = g.H, a.C = g.C;
     a.s = sign < 0 ? -1.f : 1.f;
     return a;
 }

@@ -627,11 +627,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     }
     const double us = P.Mrx / 2 + (ss - P.sb), ut = P.Mry / 2 + (ts - P.tb);  // Ds = Dt = 1
     const double fs = floor(us), ft = floor(ut);
-    const double difs = static_cast<double>(us - fs), dift = static_cast<double>(ut - ft);
+    const double difs = us - fs, dift = ut - ft;
     const int ifirst = wrap(static_cast<long long>(fs) - P.ms + P.Mrx / 2, P.Mrx);
     const int jfirst = wrap(static_cast<long long>(ft) - P.ms + P.Mry / 2, P.Mry);
     const int W = 2 * P.ms + 1;
-    const double t1 = static_cast<double>(P.t1);
+    const double t1 = P.t1;
     double res0 = 0.0, res1 = 0.0;
     const int nk = static_cast<int>(min(32LL, n - k0));
     for (int o = 0; o < nk; ++o) {
@@ -667,8 +667,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
                 for (int rr = 0; rr < rn; ++rr) {
                     const double wr = __shfl_sync(0xffffffffu, wrow[m], rr);
                     const double2 v = col[static_cast<size_t>(j) * P.Mrx];
-                    s0 += static_cast<double>(v.x) * wr;
-                    s1 += static_cast<double>(v.y) * wr;
+                    s0 += v.x * wr;
+                    s1 += v.y * wr;
                     j = j + 1 == P.Mry ? 0 : j + 1;
                 }
             }
@@ -693,10 +693,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         const double arg = (ss - P.sb) * P.xb + (ts - P.tb) * P.yb;   // :189
         double sa, ca;
         sincos(arg, &sa, &ca);
-        const double a0 = static_cast<double>(res0), a1 = static_cast<double>(res1);
         double2 out;
-        out.x = ((a0 * ca + a1 * sa) * comp);
-        out.y = ((a1 * ca - a0 * sa) * comp);
+        out.x = (res0 * ca + res1 * sa) * comp;
+        out.y = (res1 * ca - res0 * sa) * comp;
         F[k] = out;
     }
 }
