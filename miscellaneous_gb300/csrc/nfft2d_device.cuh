@@ -270,6 +270,32 @@ __device__ __forceinline__ void weights_poly2(float t1, float t2, float (&w1)[2 
     weights_even<K, 2>(ts, ws, P);
 }
 
+// The taps of one dimension, a Horner run a tap (two taps per packed FMA).  More
+// FMAs than the half-degree form, but shorter chains: faster where a thread
+// forms both dimensions' 15 or 17 weights at once from the registers of 24 warps
+// an SM (the direct gather at w 7 and 8).
+template <int K>
+__device__ __forceinline__ void weights_poly(float t, float (&w)[2 * K + 1], const WinPoly &P) {
+    constexpr int D = poly_degree(K);
+    const float2 tt = make_float2(t, t);
+    float2 acc[K];
+    float last = P.c[D][2 * K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) acc[j] = *reinterpret_cast<const float2 *>(&P.c[D][2 * j]);
+#pragma unroll
+    for (int d = D - 1; d >= 0; --d) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) acc[j] = __ffma2_rn(acc[j], tt, *reinterpret_cast<const float2 *>(&P.c[d][2 * j]));
+        last = fmaf(last, t, P.c[d][2 * K]);
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        w[2 * j] = acc[j].x;
+        w[2 * j + 1] = acc[j].y;
+    }
+    w[2 * K] = last;
+}
+
 // The taps and their derivatives d/dt from the same polynomials: Horner for
 // value and slope together (slope = slope * t + value before each value
 // step), two taps per packed FMA.  The slope of the fit differs from the
