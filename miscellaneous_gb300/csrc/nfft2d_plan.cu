@@ -828,11 +828,15 @@ __global__ void k_bin_gather(const RecT *tmp, const int *src, int M, RecT *recs)
 // Binning of one small point set in one cooperative launch: the passes above
 // with grid barriers for launch boundaries.  The points stay in their threads'
 // registers from the reduction to their sorted place, and the per-tile counts
-// that place cells and work items are added up beside the cells' own.  Bound
-// by three barriers (1.5 us each) and a round trip to L2 per phase; as two
-// fills and five launches it was bound by the launches.  The counts that the
-// host needs are written to page-locked memory, not copied there.  set_points
-// with its read-back, 4096 points on 128^2 cells: 41 -> 23 us.
+// that place cells and work items are added up beside the cells' own, one
+// addition a tile and warp.  Their counters stand apart (tile_step), as additions
+// to one line of memory wait for each other: adjacent, 131072 uniform points on
+// 256^2 cells took 41 us, 20.7 now, 21.7 in separate passes.  Up to 16 counters
+// are adjacent, half a line, so that a warp's additions go together (64^2 cells
+// 20.7, apart 24.2).  Bound by three barriers (1.5 us each) and a round trip to L2
+// per phase; as two fills and five launches it was bound by the launches.  The
+// counts that the host needs are written to page-locked memory, not copied
+// there.  set_points with its read-back, 4096 points on 128^2 cells: 41 -> 23 us.
 // ---------------------------------------------------------------------------
 constexpr int kOneBinThreads = 512, kOneBinItems = 2;
 constexpr long long kOneBinPoints = 1LL * kGridCtas * kOneBinThreads * kOneBinItems;
@@ -848,6 +852,7 @@ struct OneBinArgs {
     void *recs;
     int *src;
     unsigned *cell_count, *tile_count;
+    int tile_step;  // words from one tile's counter to the next
     int4 *chunks;
     int chunk;
     int *status;
@@ -882,7 +887,7 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, gid = blockIdx.x * kOneBinThreads + tid;
     const int ntiles = g.tiles1 * g.tiles2, cpt = g.T * g.T, ncells = ntiles * cpt;
     for (int i = gid; i < ncells; i += kStride) a.cell_count[i] = 0u;
-    if (gid < ntiles) a.tile_count[gid] = 0u;
+    if (gid < kOneBinTiles) a.tile_count[gid] = 0u;
     if (gid < 4) a.status[gid] = 0;
     grid_arrive(a.status);
     RecT r[kOneBinItems];
@@ -913,7 +918,8 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
         if (have) rank[u] = atomicAdd(a.cell_count + key[u], 1u);
         // one addition per tile and warp: the points of a dense set share it
         const unsigned t = have ? key[u] / cpt : 0xffffffffu, same = __match_any_sync(0xffffffffu, t);
-        if (have && lane == __ffs(same) - 1) atomicAdd(a.tile_count + t, static_cast<unsigned>(__popc(same)));
+        if (have && lane == __ffs(same) - 1)
+            atomicAdd(a.tile_count + t * a.tile_step, static_cast<unsigned>(__popc(same)));
     }
     if (!grid_barrier(a.status, 2, a.give_up)) return bin_one_done<RecT>(a, false);
     // where every tile's points and work items start, in each CTA: (points,
@@ -921,7 +927,7 @@ __global__ void __launch_bounds__(kOneBinThreads, 1) k_bin_one(const __grid_cons
     unsigned long long before = 0;
     for (int t0 = 0; t0 < ntiles; t0 += kOneBinThreads) {
         const int t = t0 + tid;
-        const unsigned n = t < ntiles ? __ldcg(a.tile_count + t) : 0u;
+        const unsigned n = t < ntiles ? __ldcg(a.tile_count + t * a.tile_step) : 0u;
         const unsigned long long v = static_cast<unsigned long long>(n) << 32 | (n + a.chunk - 1) / a.chunk;
         unsigned long long incl = v;
 #pragma unroll
@@ -1457,7 +1463,7 @@ int setup_bins(nfft2d_plan_s *p) {
     p->scan_tmp_elems = 2 * (scan_state_words(p->ncells + 1, kCellScanThreads * kCellScanItems) +
                              2 * scan_state_words(ntiles + 1, kItemScanThreads * kItemScanItems));
     p->tile_count_at = p->scan_tmp_elems;  // then a counter per tile (k_bin_one)
-    p->scan_tmp_elems += ntiles;
+    p->scan_tmp_elems += kOneBinTiles;
     NFFT_TRY_CUDA(plan_malloc(reinterpret_cast<void **>(&p->cell_count), sizeof(unsigned) * (p->ncells + 1)));
     NFFT_TRY_CUDA(plan_malloc(reinterpret_cast<void **>(&p->scan_tmp), sizeof(unsigned) * p->scan_tmp_elems));
     return NFFT2D_OK;
@@ -2120,16 +2126,20 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
     return status;
 }
 
-// One launch bins sets of up to 2^17 points (two a thread) on up to 2048 tiles.
-// Measured on GB300, set_points with its read-back, us, separate passes -> one
-// launch: 4096 points on 128^2 cells 41 -> 23; 16000 on 256^2 47 -> 26; 130000
-// on 512^2 49 -> 36 (all in one patch of the grid: 52 -> 39); FP64 130000 on
-// 512^2 50 -> 39.  A binning that runs beside the padding and the FFT
-// (`overlapped`) has its grid wait for their CTAs: 43 -> 28 at 4096 points, 51
-// -> 45 at 65000, but 47 -> 48 at 130000, and in FP64, whose FFT is cuFFT's,
-// 74 -> 89 and 267 -> 281; so FP32 and 2^16 points there.
-static bool use_one_bin(const nfft2d_plan_s *p, long long M, bool overlapped) {
-    return M <= kOneBinPoints && (!overlapped || (p->precision == NFFT2D_F32 && M <= kOneBinPoints / 2)) &&
+// One launch bins sets of up to 2^17 points (two a thread) on up to 2048 tiles,
+// of up to 2^16 where the host does not wait for the counts (the round trip is
+// what one launch saves most of).  Measured on GB300, us, separate passes -> one
+// launch, uniform points:
+//   set_points, with its read-back: 4096 points on 128^2 cells 36 -> 23; 65536 on
+//     256^2 36 -> 26; 131072 on 128^2 36 -> 29, on 256^2 36 -> 30, on 500^2 41 -> 35
+//   enqueued only: 4096 on 128^2 18.5 -> 12.5; 65536 on 256^2 21.5 -> 16.4; but
+//     131072 on 128^2 20.7 -> 20.6, on 80^2 24.8 -> 26.7, in a tenth of 720^2 28.9 ->
+//     30.9, in FP64 on 64^2 26.7 -> 28.8
+// A binning that runs beside the padding and the FFT (`overlapped`) has its grid
+// wait for their CTAs: 35 -> 27 at 65536 points on 256^2 cells, but in FP64, whose
+// FFT is cuFFT's, 74 -> 89 and 267 -> 281; so FP32 only there.
+static bool use_one_bin(const nfft2d_plan_s *p, long long M, bool async, bool overlapped) {
+    return M <= (async ? kOneBinPoints / 2 : kOneBinPoints) && (!overlapped || p->precision == NFFT2D_F32) &&
            1LL * p->g.tiles1 * p->g.tiles2 <= kOneBinTiles && p->chunk <= kSpreadItemMax && p->num_sms >= kGridCtas;
 }
 
@@ -2186,7 +2196,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
     const float s1f = static_cast<float>(s1), s2f = static_cast<float>(s2);
     stage_begin(p, ST_SORT);
     const int *hs = p->h_status;  // page-locked
-    const bool one = use_one_bin(p, M, coords_read != nullptr);
+    const bool one = use_one_bin(p, M, async, coords_read != nullptr);
     p->binning = one ? 2 : 1;
     if (one) {
         OneBinArgs a{};
@@ -2194,6 +2204,7 @@ int nfft2d::set_points_scaled(nfft2d_plan_s *p, long long M, const void *x1, con
         a.o1 = o1, a.o2 = o2, a.s1 = s1, a.s2 = s2, a.s1f = s1f, a.s2f = s2f, a.exact = exact;
         a.g = g;
         a.recs = p->recs, a.src = p->src, a.cell_count = p->cell_count, a.tile_count = p->scan_tmp + p->tile_count_at;
+        a.tile_step = g.tiles1 * g.tiles2 <= 16 ? 1 : std::min(32, kOneBinTiles / (g.tiles1 * g.tiles2));
         a.chunks = p->chunks, a.chunk = p->chunk;
         a.status = p->d_status;
         a.host = async ? nullptr : p->h_status;

@@ -40,6 +40,16 @@ def test_binning(N1, N2, M, tuning, want, precision):
     assert _paths(N1, N2, M, tuning, precision=precision)["binning"] == want
 
 
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("M,want", [(1 << 16, 2), ((1 << 16) + 1, 1)])
+def test_binning_without_a_wait(M, want, precision):
+    from miscellaneous_gb300.nfft import Plan
+    with Plan(64, 64, precision=precision) as p:
+        p.set_points(*_x(M), sync=False)
+        assert p.paths()["binning"] == want
+        p.synchronize()
+
+
 @pytest.mark.parametrize("M,precision,want", [(1 << 16, "f32", 2), ((1 << 16) + 1, "f32", 1), (1000, "f64", 1)])
 def test_binning_beside_the_forward(M, precision, want):
     assert _paths(64, 64, M, bin_and_forward=True, precision=precision)["binning"] == want
