@@ -22,6 +22,7 @@ def _middle(rng, n, lo, hi):
 
 @pytest.mark.parametrize("eps,M,N,scale", [
     (0.5, 300, 200, 1.0), (1e-4, 1000, 777, 3.0), (1e-6, 33, 65, 1.0), (1e-6, 20000, 30000, 0.02),
+    (1e-6, 50, 60, 8.0),  # far fewer than tiles
     (1e-6, 100000, 50000, 1.0), (1e-9, 5000, 4000, 1.0), (1e-13, 500, 300, 1.0),
 ])
 def test_f32_matches_f64(eps, M, N, scale):
