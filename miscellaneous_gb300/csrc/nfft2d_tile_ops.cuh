@@ -71,10 +71,12 @@ __device__ __forceinline__ float2 gather_direct_f32(const float2 *grid, int H, i
     constexpr int W = 2 * K + 1;
     constexpr int V = K + 1;  // float4 loads per row
     float w1[W], w2[W];
-    // Both directions' forms measured on GB300, a forward in us, 2^21 points on
-    // 2048^2, w 7 | 8: half-degree 446 | 493, Horner 443 | 483; 2^18 on 512^2: 55.9 |
-    // 57.6, 51.5 | 53.1; at w 6 the half-degree form wins, 402 -> 396.
-    if constexpr (K > 6) {
+    // Which form, measured on GB300, us: a plan's forward, 2^21 points on 2048^2, w 6 |
+    // 7 | 8, half-degree 396 | 446 | 493, Horner 402 | 443 | 483; 2^18 on 512^2, w 7 | 8,
+    // 55.9 | 57.6 and 51.5 | 53.1.  The batched gather, whose taps are loaded while the
+    // weights form, w 6: 6 transforms of 100 points 27.7 and 24.9, 8 of 4 10^5 401
+    // and 393; w 4: 22.8 and 22.8, 264.7 and 268.1.
+    if constexpr (K > (WAIT ? 6 : 5)) {
         weights_poly<K>(t1, w1, wp);
         weights_poly<K>(t2, w2, wp);
     } else {
