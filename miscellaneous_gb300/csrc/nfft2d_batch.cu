@@ -672,7 +672,7 @@ int nfft2d_batch_destroy(nfft2d_batch b) {
 }
 
 // far: the far-field step's points -- device memory, scaled by c1 and c2 first;
-// NFFT2D_ERR_UNSUPPORTED when they don't bin in one launch.
+// only if they bin in one launch (small_bin_takes).
 static int batch_set_points(nfft2d_batch b, const long long *M, const void *const *x1, const void *const *x2,
                             int coord_dtype, int units, bool far, float c1, float c2) {
     b->points_valid = false;
@@ -775,7 +775,9 @@ int nfft2d_batch_far_field(nfft2d_batch b, long long M, const float *const *X, c
     if (!b || !X || !Y || !excitations || !far_field || M < 0 || M > 0x7fffffffLL) return NFFT2D_ERR_INVALID_ARG;
     const int n = b->count;
     long long cells = -1;
+    bool small = true;
     for (int i = 0; i < n; ++i) {
+        small = small && small_bin_takes(b->plans[i], M);
         const long long c = static_cast<long long>(b->plans[i]->N1) * b->plans[i]->N2;
         if (cells >= 0 && c != cells && filter) return NFFT2D_ERR_INVALID_ARG;  // one filter for one grid size
         cells = c;
@@ -788,9 +790,13 @@ int nfft2d_batch_far_field(nfft2d_batch b, long long M, const float *const *X, c
     // fields as it writes them: no pass of their own
     const std::vector<long long> Ms(static_cast<size_t>(n), M);
     std::vector<const void *> px(X, X + n), py(Y, Y + n);
-    int st = batch_set_points(b, Ms.data(), px.data(), py.data(), NFFT2D_COORD_F32, NFFT2D_UNITS_GRID, true, scale_x,
+    int st = NFFT2D_OK;
+    if (small) {
+        st = batch_set_points(b, Ms.data(), px.data(), py.data(), NFFT2D_COORD_F32, NFFT2D_UNITS_GRID, true, scale_x,
                               scale_y);
-    if (st == NFFT2D_ERR_UNSUPPORTED) {  // larger sets: scaled copies, binned per transform
+    } else {  // larger sets: scaled copies, binned per transform
+        // (allocated before batch_set_points waits for the stream: at a wait the
+        // pool gives freed memory back, and it would be mapped again on each call)
         float *xs = nullptr, *ys = nullptr;
         const float **dxy = nullptr;
         const size_t pts = static_cast<size_t>(n) * static_cast<size_t>(M);
@@ -799,7 +805,6 @@ int nfft2d_batch_far_field(nfft2d_batch b, long long M, const float *const *X, c
         B_TRY(cudaMallocAsync(&dxy, sizeof(float *) * 2 * n, b->stream));
         std::vector<const void *> hxy(px);
         hxy.insert(hxy.end(), py.begin(), py.end());
-        st = NFFT2D_OK;
         if (cudaMemcpyAsync(dxy, hxy.data(), sizeof(float *) * 2 * n, cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
             st = NFFT2D_ERR_CUDA;
         if (st == NFFT2D_OK && M > 0) {

@@ -276,6 +276,9 @@ struct SmallBinSpace {
     int *h_out = nullptr;                              // 2 a transform, page-locked, written by the kernel
 };
 
+// Whether bin_small_batch takes M points of this plan.
+bool small_bin_takes(const nfft2d_plan_s *p, long long M);
+
 // Bin the points of `count` FP32 plans (a batch's transforms) with one
 // launch: one CTA per transform with its cell counters in shared memory.
 // Same result as nfft2d_set_points on each plan (units: NFFT2D_UNITS_*);

@@ -2039,6 +2039,14 @@ static int coord_device_ptr(const nfft2d_plan_s *p, const void *x, const void **
 }
 
 extern "C++" {
+// the counters must fit in shared memory
+static size_t small_bin_smem(size_t cells) { return sizeof(unsigned) * (cells + 1 + 32); }
+constexpr int kSmallBinSmem = 200 * 1024;
+
+bool nfft2d::small_bin_takes(const nfft2d_plan_s *p, long long M) {
+    return p->precision == NFFT2D_F32 && M <= (1LL << 24) && small_bin_smem(p->ncells) <= kSmallBinSmem;
+}
+
 int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, const void *const *x1,
                              const void *const *x2, int coord_dtype, int units, int count, cudaStream_t stream,
                              const SmallBinSpace &space, float c1, float c2, bool device_coords) {
@@ -2049,13 +2057,11 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
     size_t max_cells = 0;
     for (int i = 0; i < count; ++i) {
         nfft2d_plan_s *p = plans[i];
-        if (!p || M[i] < 0 || M[i] > (1LL << 24) || p->precision != NFFT2D_F32) return NFFT2D_ERR_UNSUPPORTED;
+        if (!p || M[i] < 0 || !small_bin_takes(p, M[i])) return NFFT2D_ERR_UNSUPPORTED;
         if (M[i] > 0 && (!x1[i] || !x2[i])) return NFFT2D_ERR_INVALID_ARG;
         max_cells = std::max(max_cells, p->ncells);
     }
-    const size_t smem = sizeof(unsigned) * (max_cells + 1 + 32);
-    constexpr int kMost = 200 * 1024;
-    if (smem > kMost) return NFFT2D_ERR_UNSUPPORTED;  // the counters must fit in shared memory
+    const size_t smem = small_bin_smem(max_cells);
     for (int i = 0; i < count; ++i) {
         nfft2d_plan_s *p = plans[i];
         const void *dx1 = x1[i], *dx2 = x2[i];
@@ -2103,7 +2109,7 @@ int nfft2d::bin_small_batch(nfft2d_plan_s *const *plans, const long long *M, con
     }
     NFFT_TRY_CUDA(cudaMemcpyAsync(space.d_jobs, space.h_jobs, sizeof(SmallBinJob) * count, cudaMemcpyHostToDevice, stream));
     auto kernel = coord_dtype == NFFT2D_COORD_F64 ? k_bin_small<double> : k_bin_small<float>;
-    NFFT_TRY_CUDA(allow_smem(kernel, static_cast<int>(smem), kMost));
+    NFFT_TRY_CUDA(allow_smem(kernel, static_cast<int>(smem), kSmallBinSmem));
     kernel<<<count, kSmallBinThreads, smem, stream>>>(space.d_jobs);
     NFFT_TRY_CUDA(cudaGetLastError());
     NFFT_TRY_CUDA(cudaStreamSynchronize(stream));
