@@ -470,6 +470,18 @@ cudaError_t launch(Kernel kernel, const nfft2d_plan_s *p, bool after, int blocks
 
 }  // namespace
 
+// Below 2048 x 2048 cells, and above where both sides have a prime factor of 5 or
+// more (powers of 2 and 3 are what cuFFT is best at).  Measured on GB300, w 6, 50 k
+// points, coefficients, us, cuFFT with its separate kernels -> here (forward |
+// adjoint):
+//     50 x 50    25.5 -> 18.9 | 41.3 -> 39.0      250 x 378   36.9 -> 27.1 | 45.2 -> 37.0
+//    500 x 500   39.0 -> 34.9 | 53.4 -> 49.9      630 x 630   66.6 -> 53.3 | 81.7 -> 71.8
+//   1100 x 900    136 -> 96   |  153 -> 116      1000 x 1000   120 -> 98   |  131 -> 124
+//   1100 x 1300   222 -> 137  |  234 -> 165      1920 x 1920   366 -> 306  |  394 -> 384
+//   1536 x 1536   241 -> 231  |  234 -> 254      1050 x 1024   111 -> 107  |  127 -> 134
+//   1024 x 1024    94 -> 100  |  111 -> 126      2048 x 2048   274 -> 362  |  320 -> 462
+// (the last four stay with cuFFT).  Errors fall, 2.5e-7 .. 3.7e-7 -> 2.0e-7.
+//
 // A prime above 13 costs its own length per element: up to 2^20 cells it beats
 // cuFFT's chirp transforms.  Measured on GB300, w 6, 50 k points, coefficients
 // (primes), us, cuFFT -> here (forward | adjoint):
@@ -481,7 +493,13 @@ bool mixed_fft_eligible(int precision, int n1, int n2) {
         MixedFft f;
         return n >= 64 && n <= kMixedMaxSide && factor(n, &f) && (f.radix[0] <= 16 || 1LL * n1 * n2 <= 1 << 20);
     };
-    return precision == NFFT2D_F32 && side(n1) && side(n2);
+    auto rest = [](int n) {
+        for (const int f : {2, 3})
+            while (n % f == 0) n /= f;
+        return n;
+    };
+    return precision == NFFT2D_F32 && side(n1) && side(n2) &&
+           (1LL * n1 * n2 < 2048LL * 2048LL || (rest(n1) > 1 && rest(n2) > 1));
 }
 
 cudaError_t mixed_type2_cols(const nfft2d_plan_s *p, int sign, const void *F) {

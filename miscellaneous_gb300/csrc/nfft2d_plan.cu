@@ -369,27 +369,9 @@ bool use_fused(const nfft2d_plan_s *p) {
 }
 
 // The same passes with sides of small prime factors (nfft2d_fft_mixed.cu), in
-// automatic mode, where the fused ones do not run: below 2048 x 2048 cells,
-// and above where both sides have a prime factor of 5 or more (powers of 2 and
-// 3 are what cuFFT is best at).  Not for a regridder's plan (no strips), which
-// pads by itself.  Measured on GB300, w 6, 50 k points, coefficients, us, cuFFT
-// with its separate kernels -> here (forward | adjoint):
-//     50 x 50    25.5 -> 18.9 | 41.3 -> 39.0      250 x 378   36.9 -> 27.1 | 45.2 -> 37.0
-//    500 x 500   39.0 -> 34.9 | 53.4 -> 49.9      630 x 630   66.6 -> 53.3 | 81.7 -> 71.8
-//   1100 x 900    136 -> 96   |  153 -> 116      1000 x 1000   120 -> 98   |  131 -> 124
-//   1100 x 1300   222 -> 137  |  234 -> 165      1920 x 1920   366 -> 306  |  394 -> 384
-//   1536 x 1536   241 -> 231  |  234 -> 254      1050 x 1024   111 -> 107  |  127 -> 134
-//   1024 x 1024    94 -> 100  |  111 -> 126      2048 x 2048   274 -> 362  |  320 -> 462
-// (the last four stay with cuFFT).  Errors fall, 2.5e-7 .. 3.7e-7 -> 2.0e-7.
-bool use_mixed(const nfft2d_plan_s *p) {
-    if (!p->mixed_ok || p->fft_mode >= 0 || use_fused(p)) return false;
-    auto rest = [](int n) {
-        for (const int f : {2, 3})
-            while (n % f == 0) n /= f;
-        return n;
-    };
-    return 1LL * p->g.n1 * p->g.n2 < 2048LL * 2048LL || (rest(p->g.n1) > 1 && rest(p->g.n2) > 1);
-}
+// automatic mode, where the fused ones do not run.  Not for a regridder's plan
+// (no strips), which pads by itself.
+bool use_mixed(const nfft2d_plan_s *p) { return p->mixed_ok && p->fft_mode < 0 && !use_fused(p); }
 
 // Whole transforms in one launch (nfft2d_small.cu) for small sets on small
 // grids, where launches and latency are most of the time: with the plan's own
