@@ -1130,7 +1130,8 @@ def run_ours(args, wl):
                            tuning=(tuned or {}).get("tuning"), plan=plan.info()),
             "autotune_trials_ms": [{**c, "ms": round(ms, 4)} for c, ms in (tuned or {}).get("trials", [])] or None,
             "stages_ms": stage,
-            "stages_note": STAGES_NOTE[fused],
+            "stages_note": STAGES_NOTE[fused] + ("; timed a kernel a stage, where the timed steps take one launch a direction"
+                                                 if paths["forward"] or paths["adjoint"] else ""),
             "forward_ms": stage["pad"] + stage["fft_fwd"] + stage["halo_fill"] + stage["gather"],
             "adjoint_ms": stage["spread"] + stage["fold"] + stage["fft_adj"] + stage["crop"],
             "fft_ms": (stage["pad"] + stage["fft_fwd"] + stage["fold"] + stage["fft_adj"]) if fused
