@@ -265,8 +265,8 @@ __global__ void __launch_bounds__(kThreads, K <= 6 ? 4 : 3)
 // operand reads of the MMAs, 4 cycles a point, and the point's own weights
 // going in and out, 5 of the 12 cycles it takes an SM at w 6 (ncu, 2^23
 // clustered points: issue 48 %, load/store wavefronts 54 %); the direct gather
-// takes 16.7, bound by L1.  2^22 uniform points, w 6: 268 -> 213 us; 2^24
-// clustered: 960 -> 812 us.
+// takes 16.7, bound by L1.  2^22 uniform points, w 6: 268 -> 208 us; 2^24
+// clustered: 960 -> 790 us.
 template <int K, bool COMP>
 __global__ void __launch_bounds__(kTcPoints, kTcCtas)
     k_gather_tc(const float2 *__restrict__ grid, const Rec32 *__restrict__ recs, const int4 *__restrict__ chunks,
