@@ -209,8 +209,9 @@ int nfft2d_set_points(nfft2d_plan plan, long long M, const void *x1, const void 
  * that follow read the work-item count from device memory; x1 and x2 must
  * stay valid until the stream has run the binning.  A non-finite coordinate
  * is reported by the next nfft2d_synchronize (NFFT2D_ERR_NONFINITE, which
- * also drops the point set); transforms enqueued before that produce
- * unspecified values but stay in bounds.  nfft2d_get_info reports n_chunks
+ * also drops the point set, as NFFT2D_ERR_DEVICE_TIMEOUT of a binning that
+ * gave up does); transforms enqueued before that produce unspecified values
+ * but stay in bounds.  nfft2d_get_info reports n_chunks
  * = -1 until nfft2d_synchronize has read the count back. */
 int nfft2d_set_points_async(nfft2d_plan plan, long long M, const void *x1, const void *x2, int coord_dtype,
                             int units);
